@@ -1,0 +1,61 @@
+"""Kernels at the sizes where their tiling can go wrong (ragged tails, row and
+run lengths around a step, one domain, many nodes on one coarse level) against
+the CPU oracle or the mathematics (needs a B200)."""
+import numpy as np
+import pytest
+
+import oracle
+from agipc_learning_b200 import _native as N
+from agipc_learning_b200 import synth
+from agipc_learning_b200.solver import MasPcg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nt", [1, 31, 32, 33, 129])
+def test_element_kernel_tet_counts(nt):
+    """Whole and ragged warps of tets, a third of them inverted: triplets
+    bit-exact, values to 1e-9 of each tet's largest entry (the bound of the
+    full-size test), nothing written past the last tet."""
+    import torch
+    X, tets = synth.box_mesh(5, 5, 5, 0.01)
+    rng = np.random.default_rng(nt)
+    x = X + 0.7 * 0.01 * rng.uniform(-1, 1, X.shape)
+    tets = tets[rng.permutation(len(tets))[:nt]]
+    Di, vol, u, r = oracle.fem_rest_data(tets, X, np.full(nt, 1e5), 0.45)
+    g0, R0, C0, V0 = oracle.fem_snk1(tets, x, Di, vol, u, r, 0.01, 3)
+    D = lambda a, t: torch.from_numpy(np.ascontiguousarray(a, t)).cuda()  # noqa: E731
+    rows = torch.full((10 * nt + 32,), -7, dtype=torch.int32, device="cuda")
+    cols = rows.clone()
+    vals = torch.full((10 * nt + 32, 9), np.nan, dtype=torch.float64, device="cuda")
+    grad = torch.zeros(x.size, dtype=torch.float64, device="cuda")
+    a = [D(tets, np.int32), D(x, np.float64), D(Di, np.float64), D(vol, np.float64), D(u, np.float64), D(r, np.float64)]
+    p = [t.data_ptr() for t in a]
+    torch.cuda.synchronize()
+    with MasPcg() as m:
+        N.check(m.lib.maspcg_fem_snk1_gradient_hessian(m.h, nt, p[0], len(X), p[1], p[2], p[3], p[4], p[5], 0.01, 3,
+                                                       grad.data_ptr(), rows.data_ptr(), cols.data_ptr(),
+                                                       vals.data_ptr()), m.h)
+    R, C, V = rows.cpu().numpy(), cols.cpu().numpy(), vals.cpu().numpy()
+    assert np.array_equal(R[:10 * nt], R0) and np.array_equal(C[:10 * nt], C0)
+    assert np.all(R[10 * nt:] == -7) and np.all(C[10 * nt:] == -7) and np.all(np.isnan(V[10 * nt:]))
+    d = np.abs(V[:10 * nt] - V0).reshape(nt, 90).max(axis=1)
+    assert np.all(d <= 1e-9 * np.abs(V0).reshape(nt, 90).max(axis=1))
+    assert np.abs(grad.cpu().numpy().reshape(-1) - g0.reshape(-1)).max() <= 1e-10 * np.abs(g0).max()
+
+
+def test_element_kernel_degenerate_tets():
+    """Rest state, a flattened, a collapsed and a huge tet: finite values that
+    match the eigendecomposition to 1e-9 (repeated and zero singular values)."""
+    X = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1.0]])
+    tets = np.array([[0, 1, 2, 3]], np.int32)
+    Di, vol, u, r = oracle.fem_rest_data(tets, X, np.full(1, 1e3), 0.4)
+    shapes = [np.eye(3), np.diag([1.0, 1.0, 0.0]), np.diag([1.0, 0.0, 0.0]), np.zeros((3, 3)), 1e3 * np.eye(3),
+              np.diag([1.0, 1.0, -1.0]), 1e-9 * np.eye(3)]
+    with MasPcg() as m:
+        for F in shapes:
+            x = X @ F.T
+            _, _, _, V0 = oracle.fem_snk1(tets, x, Di, vol, u, r, 0.1)
+            _, _, _, V1 = m.fem_snk1(tets, x, Di, vol, u, r, 0.1)
+            assert np.all(np.isfinite(V1)), F
+            assert np.abs(V1 - V0).max() <= 1e-9 * np.abs(V0).max(), F
