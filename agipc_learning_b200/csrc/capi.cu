@@ -179,7 +179,7 @@ void copy_back(maspcg_handle* h, T* user, const T* dev, size_t count)
 }  // namespace
 
 namespace {
-// Validate a coarse mapping on host copies and stage its arrays on the device.
+// Stage a coarse mapping's arrays on the device and validate them there.
 maspcg::GalerkinMap galerkin_map(maspcg_handle* h, const maspcg_galerkin_map* map)
 {
   MREQ(map != nullptr, MASPCG_ERR_INVALID_ARGUMENT, "null mapping");
@@ -190,19 +190,6 @@ maspcg::GalerkinMap galerkin_map(maspcg_handle* h, const maspcg_galerkin_map* ma
   MREQ((long long)g.prefix_blocks + g.fem_nodes <= 0x7fffffffLL &&
            (long long)g.prefix_blocks + g.coarse_block_nodes <= 0x7fffffffLL,
        MASPCG_ERR_CAPACITY, "block count overflow");
-  if (g.fem_nodes > 0) {
-    const std::vector<int> f2c = host_copy(h, g.fine_to_coarse, (size_t)g.fem_nodes);
-    const std::vector<int> base = host_copy(h, g.coarse_block_bases, (size_t)g.coarse_nodes);
-    const std::vector<int> mask = host_copy(h, g.basis_masks, (size_t)g.coarse_nodes);
-    for (int c : f2c) MREQ(c >= 0 && c < g.coarse_nodes, MASPCG_ERR_INVALID_ARGUMENT, "fine_to_coarse out of range");
-    for (int c = 0; c < g.coarse_nodes; ++c) {
-      MREQ(mask[c] >= 1 && mask[c] <= 15, MASPCG_ERR_INVALID_ARGUMENT, "basis mask outside 1..15");
-      int w = 0;
-      for (int q = 0; q < 4; ++q) w += (mask[c] >> q) & 1;
-      MREQ(base[c] >= 0 && (long long)base[c] + w <= g.coarse_block_nodes, MASPCG_ERR_INVALID_ARGUMENT,
-           "coarse block base out of range");
-    }
-  }
   maspcg::GalerkinMap m{};
   m.prefix = g.prefix_blocks;
   m.fine_blocks = g.prefix_blocks + g.fem_nodes;
@@ -211,6 +198,11 @@ maspcg::GalerkinMap galerkin_map(maspcg_handle* h, const maspcg_galerkin_map* ma
     m.coarse_block_bases = device_in(h, g.coarse_block_bases, (size_t)g.coarse_nodes, h->gal_bases);
     m.basis_masks = device_in(h, g.basis_masks, (size_t)g.coarse_nodes, h->gal_masks);
     m.rest = device_in(h, g.rest_positions, 3 * (size_t)g.fem_nodes, h->gal_rest);
+    const int broken = maspcg::galerkin_check(h, m, g.fem_nodes, g.coarse_nodes, g.coarse_block_nodes);
+    MREQ(broken == 0, MASPCG_ERR_INVALID_ARGUMENT,
+         broken == 1   ? "fine_to_coarse out of range"
+         : broken == 2 ? "basis mask outside 1..15"
+                       : "coarse block base out of range");
   }
   return m;
 }
@@ -919,13 +911,8 @@ MASPCG_API maspcg_status maspcg_bcoo_gradient(maspcg_handle* h, const int* rows,
     const size_t n = 3 * (size_t)h->nb;
     const int* r = device_in(h, rows, (size_t)n_blocks, h->adj_rows);
     const int* c = device_in(h, cols, (size_t)n_blocks, h->adj_cols);
-    // block indices must address the system (checked on the host copy)
-    {
-      const std::vector<int> hr = host_copy(h, rows, (size_t)n_blocks), hc = host_copy(h, cols, (size_t)n_blocks);
-      for (int t = 0; t < n_blocks; ++t)
-        MREQ(hr[t] >= 0 && hr[t] < h->nb && hc[t] >= 0 && hc[t] < h->nb, MASPCG_ERR_INVALID_ARGUMENT,
-             "block index outside the system");
-    }
+    MREQ(maspcg::block_indices_in_range(h, r, c, n_blocks, h->nb), MASPCG_ERR_INVALID_ARGUMENT,
+         "block index outside the system");
     const double* l = device_in(h, lam, n, h->adj_lam);
     const double* xv = device_in(h, x, n, h->adj_x);
     if (is_device_ptr(grad9)) {
@@ -953,15 +940,11 @@ MASPCG_API maspcg_status maspcg_element_modulus_gradient(maspcg_handle* h, int n
     MREQ(rows && cols && values9 && lam && x && youngs && grad_youngs, MASPCG_ERR_INVALID_ARGUMENT, "null argument");
     const size_t nblk = (size_t)n_tets * blocks_per_tet;
     MREQ(nblk <= (size_t)0x7fffffff, MASPCG_ERR_CAPACITY, "too many blocks");
-    {
-      const std::vector<int> hr = host_copy(h, rows, nblk), hc = host_copy(h, cols, nblk);
-      for (size_t t = 0; t < nblk; ++t)
-        MREQ(hr[t] >= 0 && hr[t] < h->nb && hc[t] >= 0 && hc[t] < h->nb, MASPCG_ERR_INVALID_ARGUMENT,
-             "block index outside the system");
-    }
     const size_t n = 3 * (size_t)h->nb;
     const int* r = device_in(h, rows, nblk, h->adj_rows);
     const int* c = device_in(h, cols, nblk, h->adj_cols);
+    MREQ(maspcg::block_indices_in_range(h, r, c, (long long)nblk, h->nb), MASPCG_ERR_INVALID_ARGUMENT,
+         "block index outside the system");
     DBuf<double> vstage{false}, estage{false};
     const double* v = device_in(h, values9, 9 * nblk, vstage);
     const double* l = device_in(h, lam, n, h->adj_lam);

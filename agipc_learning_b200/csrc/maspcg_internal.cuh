@@ -333,6 +333,10 @@ void solve(maspcg_handle* h, const double* b_dev, double* x_dev, maspcg_result* 
 void spmv_working(maspcg_handle* h, const double* x_int, double* y_int);  // internal order, FP64 in/out
 
 // adjoint.cu (device pointers, caller's row order)
+// Whether every block's row and column lie in [0, nb), checked on the device
+// (the arrays are there already; copying them back to look took longer than
+// the gradient).  Synchronises the stream.
+bool block_indices_in_range(maspcg_handle* h, const int* rows, const int* cols, long long n, int nb);
 void bcoo_gradient(maspcg_handle* h, const int* rows, const int* cols, int n, const double* lam, const double* x,
                    double* grad);
 void modulus_gradient(maspcg_handle* h, const int* rows, const int* cols, const double* vals, int ntet, int bpt,
@@ -370,6 +374,10 @@ struct GalerkinMap {
   int prefix;
   int fine_blocks;
 };
+// Checks a mapping on the device: 0, or the first rule broken (1: an owner
+// outside [0, coarse_nodes), 2: a mask outside 1..15, 3: a block base out of
+// range).  Synchronises the stream.
+int galerkin_check(maspcg_handle* h, const GalerkinMap& m, int fem_nodes, int coarse_nodes, int coarse_block_nodes);
 int galerkin_expand(maspcg_handle* h, const GalerkinMap& m, const double* vals, const int* rows, const int* cols,
                     int n, const double** v, const int** r, const int** c);
 void galerkin_restrict(maspcg_handle* h, const GalerkinMap& m, const double* fine, double* coarse, int coarse_blocks);

@@ -59,3 +59,30 @@ def test_element_kernel_degenerate_tets():
             _, _, _, V1 = m.fem_snk1(tets, x, Di, vol, u, r, 0.1)
             assert np.all(np.isfinite(V1)), F
             assert np.abs(V1 - V0).max() <= 1e-9 * np.abs(V0).max(), F
+
+
+@pytest.mark.parametrize("n", [1, 33, 2049])
+def test_block_gradient_checks_every_index(n):
+    """An index outside the system in the last block is refused before anything
+    is written; without it the ragged tail is written in full."""
+    import torch
+    s = synth.cube_system(4, E=1e5, seed=3)
+    rng = np.random.default_rng(n)
+    r = rng.integers(0, s.nb, n).astype(np.int32)
+    c = rng.integers(0, s.nb, n).astype(np.int32)
+    lam, x = rng.standard_normal(3 * s.nb), rng.standard_normal(3 * s.nb)
+    D = lambda a: torch.from_numpy(a).cuda()  # noqa: E731
+    with MasPcg(preconditioner="none") as m:
+        m.set_matrix(s.vals, s.rows, s.cols, s.nb)
+        out = torch.full((n, 9), 5.0, dtype=torch.float64, device="cuda")
+        for bad in (s.nb, -1):
+            rb = r.copy()
+            rb[-1] = bad
+            with pytest.raises(RuntimeError):
+                m.bcoo_gradient(D(rb), D(c), D(lam), D(x), out)
+            assert bool((out == 5.0).all())
+        m.bcoo_gradient(D(r), D(c), D(lam), D(x), out)
+    L, X = lam.reshape(-1, 3), x.reshape(-1, 3)
+    g = -L[r][:, :, None] * X[c][:, None, :]
+    g -= np.where((r != c)[:, None, None], X[r][:, :, None] * L[c][:, None, :], 0.0)
+    assert np.allclose(out.cpu().numpy(), g.transpose(0, 2, 1).reshape(-1, 9), rtol=1e-14, atol=1e-14)
