@@ -61,6 +61,21 @@ def test_element_kernel_degenerate_tets():
             assert np.abs(V1 - V0).max() <= 1e-9 * np.abs(V0).max(), F
 
 
+@pytest.mark.parametrize("n,run", [(2, 1), (31, 2), (255, 3), (257, 4), (2303, 5), (2305, 9)])
+def test_merge_run_lengths(n, run):
+    """Runs around the four-ahead fetch and element counts around a CTA:
+    bit-exact (sums in input order)."""
+    rng = np.random.default_rng(n)
+    k = (n + run - 1) // run
+    key = rng.permutation(np.repeat(np.arange(k), run)[:n])
+    r, c = (key % 53).astype(np.int32), (53 + key // 53).astype(np.int32)
+    v = rng.standard_normal((n, 9))
+    ro, co, vo = oracle.convert_triplets(r, c, v)
+    with MasPcg() as m:
+        rg, cg, vg = m.convert_bcoo(r, c, v)
+    assert np.array_equal(rg, ro) and np.array_equal(cg, co) and np.array_equal(vg, vo)
+
+
 @pytest.mark.parametrize("n", [1, 33, 2049])
 def test_block_gradient_checks_every_index(n):
     """An index outside the system in the last block is refused before anything
