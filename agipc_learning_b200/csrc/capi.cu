@@ -442,8 +442,6 @@ MASPCG_API maspcg_status maspcg_set_graph(maspcg_handle* h, int vert_num, int co
     h->nlist.resize(std::max(neighbor_list_size, 1));
     up(h->pmr, pmr);
     up(h->rmp, rmp);
-    h->h_pmr = pmr;
-    h->h_rmp = rmp;
     const int L = h->levelnum;
     h->fine_mask.resize(vert_num);
     h->next_mask.resize(vert_num);

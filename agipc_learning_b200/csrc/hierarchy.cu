@@ -122,12 +122,13 @@ __global__ void k_collision(uint32_t* connect, const int* __restrict__ cst_level
         conn[j] |= 1u << (my % kB);
       }
     }
+  // Only bits that are not there yet: at the coarse levels thousands of pairs
+  // meet on a few nodes, and their atomics would queue on those addresses
+  // (bits are only ever set, so a stale read costs an atomic, never a bit).
   for (int i = 0; i < cnt; ++i) {
-    if (cst_level) {
-      if (cp[i] >= 0) atomicOr(connect + cp[i], conn[i]);
-    } else {
-      if (v[i] >= 0) atomicOr(connect + v[i], conn[i]);
-    }
+    const int at = cst_level ? cp[i] : v[i];
+    if (at < 0 || conn[i] == 0u) continue;
+    if ((__ldcg(connect + at) & conn[i]) != conn[i]) atomicOr(connect + at, conn[i]);
   }
 }
 

