@@ -145,10 +145,10 @@ __global__ void k_gather_triplets(const int* __restrict__ perm, int n, const int
 
 }  // namespace
 
-int convert_bcoo(maspcg_handle* h, const int* rows, const int* cols, const double* vals, int n, int* rows_out,
-                 int* cols_out, double* vals_out)
+MergedKeys merge_keys(maspcg_handle* h, const int* rows, const int* cols, int n)
 {
-  if (n <= 0) return 0;
+  MergedKeys out{};
+  if (n <= 0) return out;
   cudaStream_t st = h->stream;
   h->asm_keys.resize(2 * (size_t)n);
   h->asm_idx.resize(2 * (size_t)n);
@@ -191,10 +191,25 @@ int convert_bcoo(maspcg_handle* h, const int* rows, const int* cols, const doubl
   const int count = last[0] + last[1];
   h->asm_start.resize((size_t)count + 1);
   k_conv_starts<<<grid, kAsmTpb, 0, st>>>(heads, pos, n, h->asm_start.get()); MLAUNCHED(h);
-  k_conv_sum<<<ceil_div(9LL * count, kAsmTpb), kAsmTpb, 0, st>>>(k1, i1, h->asm_start.get(), count, col_bits, vals,
-                                                          rows_out, cols_out, vals_out); MLAUNCHED(h);
   MCK(cudaGetLastError());
-  return count;
+  out.keys = k1;
+  out.perm = i1;
+  out.start = h->asm_start.get();
+  out.count = count;
+  out.col_bits = col_bits;
+  return out;
+}
+
+int convert_bcoo(maspcg_handle* h, const int* rows, const int* cols, const double* vals, int n, int* rows_out,
+                 int* cols_out, double* vals_out)
+{
+  const MergedKeys k = merge_keys(h, rows, cols, n);
+  if (k.count == 0) return 0;
+  k_conv_sum<<<ceil_div(9LL * k.count, kAsmTpb), kAsmTpb, 0, h->stream>>>(k.keys, k.perm, k.start, k.count, k.col_bits,
+                                                                          vals, rows_out, cols_out, vals_out);
+  MLAUNCHED(h);
+  MCK(cudaGetLastError());
+  return k.count;
 }
 
 void partition_contacts(maspcg_handle* h, const int* rows, const int* cols, const double* vals,

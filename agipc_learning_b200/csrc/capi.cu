@@ -1079,14 +1079,13 @@ MASPCG_API maspcg_status maspcg_galerkin_coarse_matrix(maspcg_handle* h, const m
     const double* v = device_in(h, values9, (size_t)9 * n, h->gal_in_vals);
     const int* r = device_in(h, rows, (size_t)n, h->gal_in_rows);
     const int* c = device_in(h, cols, (size_t)n, h->gal_in_cols);
-    const double* ev;
-    const int *er, *ec;
-    const int expanded = maspcg::galerkin_expand(h, m, v, r, c, n, &ev, &er, &ec);
-    h->gal_out_vals.resize(9 * (size_t)std::max(expanded, 1));
-    h->gal_out_rows.resize((size_t)std::max(expanded, 1));
-    h->gal_out_cols.resize((size_t)std::max(expanded, 1));
-    const int count = maspcg::convert_bcoo(h, er, ec, ev, expanded, h->gal_out_rows.get(), h->gal_out_cols.get(),
-                                           h->gal_out_vals.get());
+    const maspcg::MergedKeys k = maspcg::galerkin_keys(h, m, r, c, n);
+    const int count = k.count;
+    h->gal_out_vals.resize(9 * (size_t)std::max(count, 1));
+    h->gal_out_rows.resize((size_t)std::max(count, 1));
+    h->gal_out_cols.resize((size_t)std::max(count, 1));
+    MREQ(maspcg::galerkin_values(h, k, v, h->gal_out_rows.get(), h->gal_out_cols.get(), h->gal_out_vals.get()),
+         MASPCG_ERR_INVALID_ARGUMENT, "non-finite coarse matrix entry");
     *n_coarse = count;
     MREQ(count <= capacity, MASPCG_ERR_CAPACITY,
          "coarse output holds " + std::to_string(capacity) + " blocks, " + std::to_string(count) + " needed");

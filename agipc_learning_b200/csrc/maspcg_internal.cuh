@@ -272,10 +272,11 @@ struct maspcg_handle {
   maspcg::DBuf<unsigned long long> asm_keys, asm_types;
   maspcg::DBuf<int> asm_idx, asm_flags, asm_start, asm_rows, asm_cols, asm_rows_out, asm_cols_out;
   maspcg::DBuf<double> asm_vals, asm_vals_out;
-  // maspcg_galerkin_*: expansion counts/offsets, expanded triplets, staging
+  // maspcg_galerkin_*: expansion counts/offsets, expanded keys, sources and weights, staging
   maspcg::DBuf<int> gal_counts, gal_rows, gal_cols, gal_in_rows, gal_in_cols, gal_f2c, gal_bases, gal_masks,
       gal_out_rows, gal_out_cols;
-  maspcg::DBuf<double> gal_vals, gal_in_vals, gal_rest, gal_vec_in, gal_vec_out, gal_out_vals;
+  maspcg::DBuf<unsigned> gal_src;
+  maspcg::DBuf<double> gal_weight, gal_in_vals, gal_rest, gal_vec_in, gal_vec_out, gal_out_vals;
   // maspcg_fem_snk1_gradient_hessian host-argument staging
   maspcg::DBuf<unsigned> fem_tets;
   maspcg::DBuf<double> fem_x, fem_dminv, fem_vol, fem_len, fem_volr, fem_grad;
@@ -342,6 +343,16 @@ void modulus_gradient(maspcg_handle* h, const int* rows, const int* cols, const 
                       const double* lam, const double* x, const double* E, double* gE);
 
 // assemble.cu (device pointers; returns the unique count / the type counts)
+// The triplets' order and runs by key (row << col_bits) + col: entries
+// perm[start[u]] .. perm[start[u + 1] - 1], in input order, belong to unique key
+// u, whose key is keys[start[u]] (handle scratch).
+struct MergedKeys {
+  const unsigned long long* keys;
+  const int* perm;
+  const int* start;
+  int count, col_bits;
+};
+MergedKeys merge_keys(maspcg_handle* h, const int* rows, const int* cols, int n);
 int convert_bcoo(maspcg_handle* h, const int* rows, const int* cols, const double* vals, int n, int* rows_out,
                  int* cols_out, double* vals_out);
 void partition_contacts(maspcg_handle* h, const int* rows, const int* cols, const double* vals,
@@ -377,8 +388,10 @@ struct GalerkinMap {
 // outside [0, coarse_nodes), 2: a mask outside 1..15, 3: a block base out of
 // range).  Synchronises the stream.
 int galerkin_check(maspcg_handle* h, const GalerkinMap& m, int fem_nodes, int coarse_nodes, int coarse_block_nodes);
-int galerkin_expand(maspcg_handle* h, const GalerkinMap& m, const double* vals, const int* rows, const int* cols,
-                    int n, const double** v, const int** r, const int** c);
+// The coarse blocks' keys, then their values; galerkin_values returns false when a term is not finite.
+MergedKeys galerkin_keys(maspcg_handle* h, const GalerkinMap& m, const int* rows, const int* cols, int n);
+bool galerkin_values(maspcg_handle* h, const MergedKeys& k, const double* vals, int* rows_out, int* cols_out,
+                     double* vals_out);
 void galerkin_restrict(maspcg_handle* h, const GalerkinMap& m, const double* fine, double* coarse, int coarse_blocks);
 void galerkin_prolong(maspcg_handle* h, const GalerkinMap& m, const double* coarse, double* fine);
 
