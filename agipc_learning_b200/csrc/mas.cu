@@ -21,7 +21,7 @@
 //     blocks out and k_domain_chol16 factors them (scaled BF16/FP16 tiles);
 //   * CEMAS16: the same with 16-slot banks (48x48, FP32, 9 wrapped
 //     diagonals), with its assembly and store rules.
-// Apply (every PCG iteration): MAS32 runs the coarse levels as one dataflow
+// Apply (every PCG iteration): MAS32 runs the coarse domains as one
 // kernel beside a tensor-core level-0 apply of the 16-bit records (or a warp
 // per domain on FP32 records, each stored block used for both triangles
 // through a shuffle); CEMAS16 runs half a warp per domain (see the CEMAS16
@@ -726,42 +726,6 @@ __device__ __forceinline__ void domain_apply16(const TI* rec, unsigned char* scr
   y[2] = vf[3 * lane + 2] * back * s2;
 }
 
-// Leader of each key group gets the group sum: with kFast a butterfly when
-// the whole warp is one group (the common case at level 0: one coarse node
-// per bank), else the group's lanes in ascending order.  Both orders are
-// fixed.  (The walk over coarse levels uses the general form only: ptxas
-// fails to allocate registers for the butterfly inside that loop.)
-template <bool kFast>
-__device__ __forceinline__ void group_sum(int key, const float v[3], float out[3], bool& leader)
-{
-  const unsigned grp = __match_any_sync(kFull, key);
-  float s0, s1, s2;
-  if (kFast && grp == kFull) {  // warp-uniform
-    s0 = v[0], s1 = v[1], s2 = v[2];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      s0 += __shfl_xor_sync(kFull, s0, o);
-      s1 += __shfl_xor_sync(kFull, s1, o);
-      s2 += __shfl_xor_sync(kFull, s2, o);
-    }
-  } else {
-    s0 = s1 = s2 = 0.f;
-    for (int src = 0; src < 32; ++src) {
-      const float a0 = __shfl_sync(kFull, v[0], src), a1 = __shfl_sync(kFull, v[1], src),
-                  a2 = __shfl_sync(kFull, v[2], src);
-      if ((grp >> src) & 1u) {
-        s0 += a0;
-        s1 += a1;
-        s2 += a2;
-      }
-    }
-  }
-  out[0] = s0;
-  out[1] = s1;
-  out[2] = s2;
-  leader = (__ffs(grp) - 1) == (int)(threadIdx.x & 31);
-}
-
 // Copy a 16-bit domain record to a warp's shared-memory slot with coalesced
 // 16-byte loads (streaming: a record is read once per apply).
 __device__ __forceinline__ void stage_record(const uint4* __restrict__ src, unsigned char* slot, int lane)
@@ -780,48 +744,59 @@ constexpr int kApplyTpb = 128;
 constexpr int kDirectSmem16 = (kApplyTpb / 32) * (kRecBytes16 + kApplyScratch);
 #define MAS_APPLY_BOUNDS(TI) __launch_bounds__(kApplyTpb, 4)
 
-// ---- coarse levels in one kernel (restriction + coarse domain applies) ----
+// ---- coarse levels (restriction + coarse domain applies) -------------------
 //
-// BuildMultiLevelR and the coarse part of _schwarzLocalXSym6 as a dataflow
-// over the hierarchy.  CTA c restricts level-0 banks [16c, 16c + 16) (two
-// per warp, so one resident wave of CTAs covers them) into level-1 nodes.  A coarse domain (32 consecutive nodes of level
-// l >= 1) is complete once every unit that writes one of its nodes has
-// finished; each unit counts itself into the domains its parents fall in,
-// and the unit that completes a domain processes it in the same CTA:
-// restricts its nodes into level l + 1 (which may complete further domains)
-// and applies the domain's inverse.  Sums run in a fixed order (group sums
-// in lane order), so the result does not depend on which CTA finishes last;
-// nothing waits.  Counters return to zero as they complete.
-constexpr int kChainWarps = 8;
-constexpr int kChainBanks = 2;                          // level-0 banks each warp restricts
-constexpr int kChainUnitBanks = kChainWarps * kChainBanks;  // banks per CTA: one resident wave covers them
-constexpr int kChainQueue = 64;
-constexpr int kChainApplySlots = 4;  // 16-bit domain records staged in shared memory at a time
+// BuildMultiLevelR and the coarse part of _schwarzLocalXSym6.  Level 1's R is
+// summed from the fine residual by the kernel that forms it (the x / r update,
+// or k_restrict1); every coarse domain then runs in one launch, a CTA each,
+// with no CTA waiting on another: a domain of level l >= 3 sums the levels
+// below its own nodes again for itself (a few thousand values) instead of
+// waiting for the CTAs that own them.  32-slot banks only: with 16 the levels are
+// more and wider (6,912 level-1 nodes below one CTA at 110,592 rows), and the
+// kernel per level stays ahead of this form (75.5 against 82.9 us per iteration).
 
-// Dynamic shared memory of k_coarse_chain: 16-bit records are staged (their
-// two passes then read shared memory), FP32 records are read from global.
-template <typename TI>
-constexpr int chain_smem_bytes() { return sizeof(TI) == 2 ? kChainApplySlots * (kRecBytes16 + kApplyScratch) : 0; }
-
-// One thread counts a finished unit, whose parents span global slots
-// [lo, hi], into the parent domains; domains it completes are appended to
-// the CTA's queue (the thread's `tail`).  Release before the counts, acquire
-// after a completion.
-__device__ __forceinline__ void chain_arrive(const ApplyArgs& a, int lo, int hi, int* queue, int& tail)
+// The children of every level-l node: they lie in one bank of level l - 1 (kB
+// nodes), so a node keeps that bank and the bits of its children's lanes.
+template <int kB>
+__global__ void k_children(const int* __restrict__ going_next, int begin_prev, int count_prev, int begin_next,
+                           int* child_bank, unsigned* child_mask)
 {
-  const int d1 = a.lv.dom_begin[1];
-  __threadfence();
-  for (int g = lo / kBank; g <= hi / kBank; ++g) {
-    const int old = atomicAdd(a.chain_count + (g - d1), 1);
-    if (old + 1 == a.chain_target[g - d1]) {
-      a.chain_count[g - d1] = 0;
-      if (tail < kChainQueue)
-        queue[tail++] = g;
-      else
-        atomicExch(a.err, 2);
-    }
-  }
-  __threadfence();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if ((t & ~31) >= count_prev) return;  // whole warp past the level
+  const int lane = threadIdx.x & 31;
+  const int key = t < count_prev ? going_next[begin_prev + t] - begin_next : -1;
+  const unsigned grp = __match_any_sync(kFull, key);
+  if (key < 0 || __ffs(grp) - 1 != lane) return;
+  child_bank[key] = t / kB;
+  child_mask[key] = kB == 32 ? grp : grp >> (lane & 16);
+}
+
+struct CoarseLevels {
+  const int* child_bank[kMaxLevels];       // l >= 2
+  const unsigned* child_mask[kMaxLevels];
+  const int* going_next;
+  int2* span;                   // per coarse domain, kMaxLevels entries: [first, last) node of level m below it
+  const float* r1;              // R of level 1, 3 per node (padding zero)
+  float* scratch;               // per level l >= 3, R of the levels 2 .. l - 1 below it where it does not fit on chip
+  float* z;                     // Z of every coarse level
+  const void* inv;
+  const float* scale;
+  LevelInfo lv;
+  int c0;
+};
+constexpr int kCoarseOnChip = 512;   // nodes of one level whose R a CTA holds in shared memory
+constexpr int kCoarseStage = 11600;  // floats of a level staged at a time: 116 banks
+
+// Scratch floats of one level l >= 3: R of levels 2 .. l - 1 (16-byte runs).
+__host__ __device__ __forceinline__ size_t coarse_scratch_level(const LevelInfo& lv, int m)
+{
+  return (3 * (size_t)lv.count[m] + 3) / 4 * 4;
+}
+__host__ __device__ __forceinline__ size_t coarse_scratch(const LevelInfo& lv, int l)
+{
+  size_t n = 0;
+  for (int m = 2; m < l; ++m) n += coarse_scratch_level(lv, m);
+  return n;
 }
 
 // Level of a coarse domain g.
@@ -832,196 +807,300 @@ __device__ __forceinline__ int domain_level(const LevelInfo& lv, int g)
   return l;
 }
 
-// pair: the level-0 apply runs concurrently and leaves the coarse correction
-// to the p update; this kernel then also sums r.z of the coarse levels,
-// sum over domains of R.Z (= r . P Z), and completes r.z with the level-0
-// part (rz_part_done, mode as in rz_update).
-template <typename TI, typename Tv, bool kFused>
-__global__ void __launch_bounds__(kChainWarps * 32) k_coarse_chain(ApplyArgs a, const Tv* __restrict__ r,
-                                                                  PcgScalars* s, int mode, int pair, FusedArgs fa)
+// The nodes of every level below a coarse domain of level l >= 2, down to level
+// 1 (whole banks: a span may hold a few nodes of a neighbouring domain).
+template <int kB>
+__global__ void k_coarse_spans(CoarseLevels a)
 {
-  __shared__ int queue[kChainQueue];
-  __shared__ int tail_s, lo_s, hi_s;
-  pdl_wait();
-  if (s && s->status != MASPCG_SOLVE_RUNNING) return;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
-    tail_s = 0;
-    lo_s = INT_MAX;
-    hi_s = -1;
-  }
-  __syncthreads();
-  FusedScal fs{};
-  if constexpr (kFused) fs = fused_scalars(s);
-  // level 0 -> level 1 (RestrictR of the fine residual); a level-1 node's
-  // children all lie in one bank, so its sum is written, not accumulated
-#pragma unroll
-  for (int k = 0; k < kChainBanks; ++k) {
-    const int bank = blockIdx.x * kChainUnitBanks + k * kChainWarps + w;
-    if (bank < a.c0 / kBank) {
-      const int slot = bank * kBank + lane;
-      const int key = a.cmap1[slot];
-      float v[3];
-      if constexpr (kFused) {
-        // r' of the iteration's update, formed as the level-0 apply forms it
-        fused_input_row(fa, fs, a.fem_off + slot, false, v);
-      } else {
-        const Tv* rp = r + 3 * (size_t)(a.fem_off + slot);
-        v[0] = (float)rp[0];
-        v[1] = (float)rp[1];
-        v[2] = (float)rp[2];
-      }
-      float o[3];
-      bool leader;
-      group_sum<true>(key >= 0 ? key : -1 - lane, v, o, leader);
-      if (leader && key >= 0) {
-        float* d = a.coarse_r + 3 * (size_t)key;
-        d[0] = o[0];
-        d[1] = o[1];
-        d[2] = o[2];
-      }
-      const int lo = (int)__reduce_min_sync(kFull, key >= 0 ? (unsigned)key : 0x7fffffffu);
-      const int hi = (int)__reduce_max_sync(kFull, key >= 0 ? (unsigned)key : 0u);
-      const bool any = __any_sync(kFull, key >= 0);  // every lane votes
-      if (lane == 0 && any) {
-        atomicMin(&lo_s, a.c0 + lo);
-        atomicMax(&hi_s, a.c0 + hi);
-      }
-    }
-  }
-  pdl_trigger();
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0 && hi_s >= 0) {
-    int t = 0;
-    chain_arrive(a, lo_s, hi_s, queue, t);
-    tail_s = t;
-  }
-  __syncthreads();
-  const int tail0 = tail_s;
-  if (tail0 == 0) return;
-  // warp 0: walk up the levels, restricting every completed domain.  Lane 0
-  // owns the queue tail; the loop bound is broadcast from it every step so
-  // the warp never diverges on it.
-  if (w == 0) {
-    int t = tail0;  // meaningful in lane 0
-    for (int i = 0; i < __shfl_sync(kFull, t, 0); ++i) {
-      const int g = queue[i];
-      const int l = domain_level(a.lv, g);
-      if (l + 1 >= a.lv.levelnum) continue;  // top level: nothing above
-      const int sg = g * kBank + lane;         // global slot of the node
-      const bool valid = sg - a.lv.begin[l] < a.lv.count[l];
-      float v[3] = {0.f, 0.f, 0.f};
-      int key = -1 - lane;
-      if (valid) {
-        const float* src = a.coarse_r + 3 * (size_t)(sg - a.c0);
-        v[0] = __ldcg(src);
-        v[1] = __ldcg(src + 1);
-        v[2] = __ldcg(src + 2);
-        key = a.going_next[sg];
-      }
-      float o[3];
-      bool leader;
-      group_sum<false>(key, v, o, leader);
-      if (leader && valid) {
-        float* d = a.coarse_r + 3 * (size_t)(key - a.c0);
-        d[0] = o[0];
-        d[1] = o[1];
-        d[2] = o[2];
-      }
-      const int lo = (int)__reduce_min_sync(kFull, valid ? (unsigned)key : 0x7fffffffu);
-      const int hi = (int)__reduce_max_sync(kFull, valid ? (unsigned)key : 0u);
-      if (lane == 0 && lo <= hi) chain_arrive(a, lo, hi, queue, t);
-      __syncwarp();
-    }
-    if (lane == 0) tail_s = t;
-  }
-  __syncthreads();
-  // apply the completed domains' inverses: 16-bit records are copied into a
-  // shared-memory slot per warp with 77 coalesced loads per lane, so the
-  // tensor-core passes read it there
-  extern __shared__ __align__(16) unsigned char chain_slots[];
-  const int n = tail_s;
-  constexpr bool kStage = sizeof(TI) == 2;
-  constexpr int kSlots = kStage ? kChainApplySlots : kChainWarps;
-  if (w < kSlots) {
-    for (int i = w; i < n; i += kSlots) {
-      const int g = queue[i];
-      const size_t base = (size_t)(kBank * g + lane - a.c0) * 3;
-      const float x[3] = {__ldcg(a.coarse_r + base), __ldcg(a.coarse_r + base + 1), __ldcg(a.coarse_r + base + 2)};
-      float y[3];
-      if constexpr (kStage) {
-        unsigned char* slot = chain_slots + (size_t)w * (kRecBytes16 + kApplyScratch);
-        stage_record(reinterpret_cast<const uint4*>(a.inv) + (size_t)g * (kRecBytes16 / 16), slot, lane);
-        const float* scg = a.scale + (size_t)g * 96 + 3 * lane;
-        const float sc[3] = {scg[0], scg[1], scg[2]};
-        domain_apply16<TI>(reinterpret_cast<const TI*>(slot), slot + kRecBytes16, sc, lane, x, y);
-      } else {
-        domain_apply(reinterpret_cast<const float*>(a.inv) + (size_t)g * kInvElems, lane, x, y);
-      }
-      a.coarse_z[base] = y[0];
-      a.coarse_z[base + 1] = y[1];
-      a.coarse_z[base + 2] = y[2];
-      if (pair && s) {
-        // this domain's R.Z; the warp applying the last coarse domain adds
-        // them up in domain order and completes r.z
-        const int d1 = a.lv.dom_begin[1], nd = a.lv.domains - d1;
-        const double dz = warp_sum((double)x[0] * y[0] + (double)x[1] * y[1] + (double)x[2] * y[2]);
-        int last = 0;
-        if (lane == 0) {
-          a.chain_dot[g - d1] = dz;
-          __threadfence();
-          last = atomicAdd(&s->tickets[kTicketCoarse], 1u) == (unsigned)nd - 1u;
-        }
-        if (__shfl_sync(kFull, last, 0)) {
-          __threadfence();
-          double t = 0.0;
-          for (int q = lane; q < nd; q += 32) t += __ldcg(a.chain_dot + q);
-          t = warp_sum(t);
-          if (lane == 0) {
-            s->tickets[kTicketCoarse] = 0u;
-            rz_part_done(s, 1, t, mode);
-          }
-        }
-      }
-    }
+  const int g = a.lv.dom_begin[1] + blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= a.lv.domains) return;
+  const int l = domain_level(a.lv, g);
+  int2* span = a.span + (size_t)(g - a.lv.dom_begin[1]) * kMaxLevels;
+  int lo = kB * g - a.lv.begin[l], hi = min(lo + kB, a.lv.count[l]);
+  span[l] = make_int2(lo, hi);
+  for (int m = l; m >= 2; --m) {
+    lo = kB * a.child_bank[m][lo];
+    hi = min(a.lv.count[m - 1], kB * (a.child_bank[m][hi - 1] + 1));
+    span[m - 1] = make_int2(lo, hi);
   }
 }
 
-// Expected arrivals per coarse domain: the same unit/parent-range rule as
-// k_coarse_chain, counted once per build.
-__global__ void k_chain_targets(ApplyArgs a, int* target)
+// Threads of a coarse domain's CTA: a warp per 16x16 tile of a 16-bit record
+// (one 16-byte load per thread holds it), a thread per block of the wrapped
+// diagonals of an FP32 one.
+template <typename TI, int kB>
+constexpr int coarse_threads() { return sizeof(TI) == 2 ? 32 * kTiles16 : kDiags * kB; }
+
+// One coarse domain per CTA: R of its nodes, then Z = M R with the whole record
+// in registers, loaded before R is needed.  Latency is all that counts here
+// (a few hundred domains of 10-20 KB): a few dependent loads and barriers,
+// where the form before walked up the hierarchy through counters that the CTAs
+// waited on, and one warp applied a domain: 15 us for the 266 coarse domains of
+// the 64^3 system (BF16; 21.9 before), and 31.4 to 28.2 us per iteration at 8,000
+// rows, 53.5 to 43.5 at 64,000, where it is on the critical path.
+// pair: the level-0 apply runs concurrently and leaves the coarse correction
+// to the p update; this kernel then also sums r.z of the coarse levels, the
+// sum over domains of R.Z (= r . P Z), and completes r.z with the level-0
+// part (rz_part_done, mode as in rz_update).
+template <typename TI, int kB>
+__global__ void __launch_bounds__(coarse_threads<TI, kB>(), 2) k_coarse_levels(CoarseLevels a, PcgScalars* s, int mode,
+                                                                          int pair, double* dots)
 {
-  const int lane = threadIdx.x & 31;
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int d1 = a.lv.dom_begin[1];
-  const int units0 = (a.c0 / kBank + kChainUnitBanks - 1) / kChainUnitBanks;
-  int lo = 0x7fffffff, hi = -1;
-  if (gw < units0) {
-    for (int b = gw * kChainUnitBanks; b < min((gw + 1) * kChainUnitBanks, a.c0 / kBank); ++b) {
-      const int key = a.cmap1[b * kBank + lane];
-      const int l2 = (int)__reduce_min_sync(kFull, key >= 0 ? (unsigned)key : 0x7fffffffu);
-      const int h2 = (int)__reduce_max_sync(kFull, key >= 0 ? (unsigned)key : 0u);
-      const bool any = __any_sync(kFull, key >= 0);
-      if (any) {
-        lo = min(lo, a.c0 + l2);
-        hi = max(hi, a.c0 + h2);
+  constexpr int kT = coarse_threads<TI, kB>(), kN = 3 * kB;
+  constexpr bool kTiled = sizeof(TI) == 2;
+  constexpr int kD = kB / 2 + 1;  // wrapped diagonals of an FP32 record
+  // dynamic: R of the levels below (two of them), then R of a level on the way
+  // up (the partial products afterwards)
+  extern __shared__ __align__(16) float coarse_smem[];
+  float* stage = coarse_smem + 2 * 3 * kCoarseOnChip;
+  __shared__ float xs[kN], vs[kN];
+  float* p1 = stage;
+  float* p2 = stage + (kTiled ? kTiles16 * 16 : kD * kN);
+  static_assert(2 * kDiags * 3 * kBank <= kCoarseStage, "partial products share the stage");
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int g = a.lv.domains - 1 - blockIdx.x;  // the top levels, with most below them, start first
+  // the record does not change during a solve: it is fetched before the wait
+  uint4 rec;
+  float sc = 1.f, B[9];
+  const int d = tid / kB, ln = tid % kB;
+  if constexpr (kTiled) {
+    rec = __ldg(reinterpret_cast<const uint4*>(a.inv) + (size_t)g * (kRecBytes16 / 16) + tid);
+    if (tid < kN) sc = __ldg(a.scale + (size_t)g * 96 + tid);
+  } else if (d < kD) {
+    const float* src = reinterpret_cast<const float*>(a.inv) + (size_t)g * (kD * 9 * kB);
+#pragma unroll
+    for (int e = 0; e < 9; ++e) B[e] = __ldg(src + (d * 9 + e) * kB + ln);
+  }
+  pdl_wait();
+  if (s && s->status != MASPCG_SOLVE_RUNNING) return;  // uniform: nothing changes the status meanwhile
+  // ---- R
+  const int l = domain_level(a.lv, g);
+  const int2* span = a.span + (size_t)(g - a.lv.dom_begin[1]) * kMaxLevels;
+  if (l == 1) {
+    const int2 own = span[1];
+    if (tid < kN) xs[tid] = tid < 3 * (own.y - own.x) ? a.r1[3 * (size_t)own.x + tid] : 0.f;
+  } else {
+    // R of level m from level m - 1: a thread per component of a bank adds the
+    // children of each of the bank's parents in order.  What that takes besides
+    // the values (parents, child masks) does not depend on them and is loaded
+    // ahead: level 2's with the staging loads, the upper levels' at the start.
+    struct Parents {
+      int first, end;  // a bank's parents are numbered one after another
+      unsigned mask;   // children of the first (mostly the only one)
+    };
+    auto parents = [&](int m, int bank) {
+      const int* next = a.going_next + a.lv.begin[m - 1];
+      Parents t;
+      t.first = __ldg(next + kB * bank) - a.lv.begin[m];
+      t.end = kB * (bank + 1) < a.lv.count[m - 1] ? __ldg(next + kB * (bank + 1)) - a.lv.begin[m] : a.lv.count[m];
+      t.mask = __ldg(a.child_mask[m] + t.first);
+      return t;
+    };
+    auto add_children = [&](int m, const Parents& t, const float* c, int q, float* dst, const int2& to) {
+      for (int node = t.first; node < t.end; ++node) {
+        unsigned mask = node == t.first ? t.mask : __ldg(a.child_mask[m] + node);
+        float v = 0.f;
+        if (mask == (kB == 32 ? kFull : 0xffffu)) {
+#pragma unroll
+          for (int k = 0; k < kB; ++k) v += c[3 * k + q];
+        } else {
+          for (; mask; mask &= mask - 1u) v += c[3 * (__ffs(mask) - 1) + q];
+        }
+        if (node >= to.x && node < to.y) dst[3 * (node - to.x) + q] = v;
+      }
+    };
+    int2 sp[kMaxLevels];
+#pragma unroll
+    for (int m = 1; m < kMaxLevels; ++m) sp[m] = m <= l ? __ldg(span + m) : make_int2(0, 0);
+    Parents up[kMaxLevels];
+#pragma unroll
+    for (int m = 3; m < kMaxLevels; ++m)
+      if (m <= l && kB * (tid / 3) < sp[m - 1].y - sp[m - 1].x) up[m] = parents(m, sp[m - 1].x / kB + tid / 3);
+    float* far = a.scratch;
+    for (int m = 3; m < l; ++m) far += coarse_scratch(a.lv, m);
+    auto place = [&](int m) {  // where level m's R goes
+      return m == l ? xs : (sp[m].y - sp[m].x <= kCoarseOnChip ? coarse_smem + (m & 1) * 3 * kCoarseOnChip
+                                                               : far + 3 * (size_t)sp[m].x);
+    };
+    // level 2 from level 1, staged kStageBanks banks at a time with 16-byte
+    // loads (spans start at whole banks), a bank's stride padded by 16 bytes so
+    // that the sums of neighbouring banks read distinct shared-memory banks
+    constexpr int kStride = kN + 4;
+    constexpr int kStageBanks = kCoarseStage / kStride < kT / 3 ? kCoarseStage / kStride : kT / 3;
+    float* dst = place(2);
+    for (int p = sp[1].x; p < sp[1].y; p += kStageBanks * kB) {
+      const int pe = min(p + kStageBanks * kB, sp[1].y);
+      const float4* from4 = reinterpret_cast<const float4*>(a.r1 + 3 * (size_t)p);
+      const int n4 = (3 * (pe - p) + 3) / 4;  // the arrays are padded to whole 16-byte words
+#pragma unroll 6
+      for (int e = tid; e < n4; e += kT) reinterpret_cast<float4*>(stage)[e + e / (kN / 4)] = from4[e];
+      const bool mine = p + kB * (tid / 3) < pe;
+      Parents t;
+      if (mine) t = parents(2, p / kB + tid / 3);
+      __syncthreads();
+      if (mine) add_children(2, t, stage + (tid / 3) * kStride, tid % 3, dst, sp[2]);
+      __syncthreads();
+    }
+#pragma unroll
+    for (int m = 3; m < kMaxLevels; ++m) {
+      if (m > l) break;
+      const float* src = dst;
+      const int banks = (sp[m - 1].y - sp[m - 1].x + kB - 1) / kB, bank0 = sp[m - 1].x / kB;
+      far += coarse_scratch_level(a.lv, m - 1);
+      dst = place(m);
+      for (int e = tid; e < 3 * banks; e += kT)
+        add_children(m, e == tid ? up[m] : parents(m, bank0 + e / 3), src + (size_t)(e / 3) * kN, e % 3, dst, sp[m]);
+      __syncthreads();
+    }
+    if (tid >= 3 * min(kB, a.lv.count[l] - (kB * g - a.lv.begin[l])) && tid < kN) xs[tid] = 0.f;
+  }
+  if (kTiled && tid < kN) vs[tid] = xs[tid] * sc;
+  __syncthreads();
+  // ---- Z = M R
+  float y = 0.f;
+  if constexpr (kTiled) {
+    // M = S V^T V S, warp w holding tile (I, J) of V: lane 2r + h its row r,
+    // columns 8 half .. 8 half + 7 (inv16_pos swaps the halves of rows 4-7 and
+    // 12-15).  FP32 products and sums of the exactly widened elements.
+    int I = 0;
+    while ((I + 1) * (I + 2) / 2 <= w) ++I;
+    const int J = w - I * (I + 1) / 2, row = lane >> 1, half = (lane ^ (lane >> 3)) & 1;
+    const uint32_t u[4] = {rec.x, rec.y, rec.z, rec.w};
+    float V[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) V[k] = Mma16<TI>::from16((unsigned short)(u[k / 2] >> (16 * (k & 1))));
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t = fmaf(V[k], vs[16 * J + 8 * half + k], t);
+    t += __shfl_xor_sync(kFull, t, 1);
+    if ((lane & 1) == 0) p1[16 * w + row] = t;
+    __syncthreads();
+    if (tid < kN) {
+      const int R = tid >> 4;
+      float v = 0.f;
+      for (int q = 0; q <= R; ++q) v += p1[16 * (R * (R + 1) / 2 + q) + (tid & 15)];
+      vs[tid] = v;  // every warp has read its S R
+    }
+    __syncthreads();
+    t = vs[16 * I + row];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) V[k] *= t;
+    // column sums over the tile's 16 rows: halving exchanges over row bits 0,
+    // 1 and 3, then row bit 2, whose partner lane with the same half is lane ^ 9
+#pragma unroll
+    for (int n = 4; n >= 1; n >>= 1) {
+      const int mask = n == 4 ? 2 : (n == 2 ? 4 : 16);
+      const bool up = (lane & mask) != 0;
+#pragma unroll
+      for (int k = 0; k < n; ++k) {
+        const float keep = up ? V[k + n] : V[k], give = up ? V[k] : V[k + n];
+        V[k] = keep + __shfl_xor_sync(kFull, give, mask);
       }
     }
+    V[0] += __shfl_xor_sync(kFull, V[0], 9);
+    if ((lane & 8) == 0) p2[16 * w + 8 * half + ((lane & 2) << 1) + ((lane & 4) >> 1) + (lane >> 4)] = V[0];
+    __syncthreads();
+    if (tid < kN) {
+      const int C = tid >> 4;
+      for (int q = C; q < 6; ++q) y += p2[16 * (q * (q + 1) / 2 + C) + (tid & 15)];
+      y *= sc;
+    }
   } else {
-    const int g = d1 + (gw - units0);  // a coarse domain as a unit
-    if (g >= a.lv.domains) return;
-    const int l = domain_level(a.lv, g);
-    if (l + 1 >= a.lv.levelnum) return;
-    const int sg = g * kBank + lane;
-    const bool valid = sg - a.lv.begin[l] < a.lv.count[l];
-    const int key = valid ? a.going_next[sg] : 0;
-    lo = (int)__reduce_min_sync(kFull, valid ? (unsigned)key : 0x7fffffffu);
-    hi = (int)__reduce_max_sync(kFull, valid ? (unsigned)key : 0u);
-    if (!__any_sync(kFull, valid)) return;
+    // the symmetric inverse: block (ln, ln + d) serves both triangles; the
+    // products and the order of the sums are those of domain_apply
+    if (d < kD) {
+      const int c = (ln + d) & (kB - 1);
+      const float x0 = xs[3 * ln], x1 = xs[3 * ln + 1], x2 = xs[3 * ln + 2];
+      const float c0 = xs[3 * c], c1 = xs[3 * c + 1], c2 = xs[3 * c + 2];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        p1[kN * d + 3 * ln + i] = B[3 * i] * c0 + B[3 * i + 1] * c1 + B[3 * i + 2] * c2;
+        p2[kN * d + 3 * c + i] = B[i] * x0 + B[3 + i] * x1 + B[6 + i] * x2;
+      }
+    }
+    __syncthreads();
+    if (tid < kN) {
+      y = p1[tid];
+#pragma unroll
+      for (int q = 1; q < kD; ++q) {
+        y += p1[kN * q + tid];
+        y += p2[kN * q + tid];
+      }
+    }
   }
-  if (lane == 0 && hi >= 0)
-    for (int g = lo / kBank; g <= hi / kBank; ++g) atomicAdd(target + (g - d1), 1);
+  if (tid < kN) a.z[3 * (size_t)(kB * g - a.c0) + tid] = y;
+  if (!pair || !s) return;
+  double total = 0.0;
+  if (grid_finish<double, kT>(tid < kN ? (double)xs[tid] * y : 0.0, dots, blockIdx.x, gridDim.x,
+                              &s->tickets[kTicketCoarse], gridDim.x, total) &&
+      tid == 0)
+    rz_part_done(s, 1, total, mode);
+}
+
+CoarseLevels coarse_levels_args(maspcg_handle* h)
+{
+  CoarseLevels c{};
+  for (int l = 2; l < h->lv.levelnum; ++l) {
+    c.child_bank[l] = h->child_bank[l].get();
+    c.child_mask[l] = h->child_mask[l].get();
+  }
+  c.going_next = h->going_next.get();
+  c.span = reinterpret_cast<int2*>(h->coarse_span.get());
+  c.r1 = h->coarse_r.get();
+  c.scratch = h->coarse_below.get();
+  c.z = h->coarse_z.get();
+  c.inv = h->inv.get();
+  c.scale = h->cfg.inverse_storage == MASPCG_INV_FP32 ? nullptr : h->inv_scale.get();
+  c.lv = h->lv;
+  c.c0 = h->c0;
+  return c;
+}
+
+// R of level 1 from the residual on its own (a warp per 32 slots), where no
+// kernel in front summed it: the initial and standalone applies, after a
+// residual replacement, and with the fused x / r update or iteration head.
+template <typename Tv, int kB, bool kFused>
+__global__ void __launch_bounds__(kTpb) k_restrict1(ApplyArgs a, const Tv* __restrict__ r, PcgScalars* s, FusedArgs fa)
+{
+  pdl_wait();
+  if (s && s->status != MASPCG_SOLVE_RUNNING) return;
+  const int slot = blockIdx.x * kTpb + threadIdx.x;
+  if ((slot & ~31) >= a.c0) return;  // whole warp past the slots
+  FusedScal fs{};
+  if constexpr (kFused) fs = fused_scalars(s);
+  float v[3] = {0.f, 0.f, 0.f};
+  if (slot < a.c0) {
+    if constexpr (kFused) {
+      // r' of the iteration's update, formed as the level-0 apply forms it
+      fused_input_row(fa, fs, a.fem_off + slot, false, v);
+    } else {
+      const Tv* rp = r + 3 * (size_t)(a.fem_off + slot);
+      v[0] = (float)rp[0];
+      v[1] = (float)rp[1];
+      v[2] = (float)rp[2];
+    }
+  }
+  restrict_bank<kB>(slot < a.c0 ? __ldg(a.cmap1 + slot) : -1, a.coarse_r, v);
+}
+
+// The leader of each key group gets the group's sum, its lanes in ascending order.
+__device__ __forceinline__ void group_sum(int key, const float v[3], float out[3], bool& leader)
+{
+  const unsigned grp = __match_any_sync(kFull, key);
+  float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+  for (int src = 0; src < 32; ++src) {
+    const float a0 = __shfl_sync(kFull, v[0], src), a1 = __shfl_sync(kFull, v[1], src),
+                a2 = __shfl_sync(kFull, v[2], src);
+    if ((grp >> src) & 1u) {
+      s0 += a0;
+      s1 += a1;
+      s2 += a2;
+    }
+  }
+  out[0] = s0;
+  out[1] = s1;
+  out[2] = s2;
+  leader = (__ffs(grp) - 1) == (int)(threadIdx.x & 31);
 }
 
 // ---- CEMAS16 apply (MASPreconditioner::preconditioning, :2250-2291) -------
@@ -1086,7 +1165,7 @@ __global__ void __launch_bounds__(kTpb) k16_restrict(Mas16Args a, const Tv* __re
   }
   float o[3];
   bool leader;
-  group_sum<false>(parent >= 0 ? parent : -1 - (int)(threadIdx.x & 31), v, o, leader);
+  group_sum(parent >= 0 ? parent : -1 - (int)(threadIdx.x & 31), v, o, leader);
   if (parent >= 0 && leader) {
     float* d = a.coarse_r + 3 * (size_t)(parent - a.c0);
     d[0] = o[0];
@@ -1282,7 +1361,7 @@ Mas16Args make_mas16_args(maspcg_handle* h)
 // Level-0 apply + prolongation + r.z; with `partial` set, the last block
 // completes the r.z reduction over [0, total_parts) and, for mode > 0,
 // updates the PCG scalars (rz0 / beta / k).
-template <typename TI, typename Tv, typename Tacc, bool kFused>
+template <typename TI, typename Tv, typename Tacc, bool kFused, bool kLevel1>
 __global__ void MAS_APPLY_BOUNDS(TI) k_level0_apply(ApplyArgs a, const Tv* __restrict__ r, Tv* z, Tacc* partial,
                                                       int part_base, int total_parts, int mode, PcgScalars* s,
                                                       int coarse_add, int pair, FusedArgs fa, double* partial_rr)
@@ -1295,11 +1374,14 @@ __global__ void MAS_APPLY_BOUNDS(TI) k_level0_apply(ApplyArgs a, const Tv* __res
   double rr = 0.0;
   FusedScal fs{};
   if constexpr (kFused) fs = fused_scalars(s);
-  for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < a.lv.dom_begin[1]; g += warps_total) {
+  for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < a.lv.dom_begin[kLevel1 ? 2 : 1]; g += warps_total) {
     const int slot = kBank * g + lane;
-    const size_t row3 = 3 * (size_t)(a.fem_off + slot);
+    const bool level0 = !kLevel1 || g < a.lv.dom_begin[1];
+    const size_t row3 = 3 * (size_t)(level0 ? a.fem_off + slot : slot - a.c0);
     Tv r0, r1, r2;
-    if constexpr (kFused) {
+    if (!level0) {
+      r0 = a.coarse_r[row3], r1 = a.coarse_r[row3 + 1], r2 = a.coarse_r[row3 + 2];
+    } else if constexpr (kFused) {
       float rn[3];
       fused_input_row(fa, fs, a.fem_off + slot, true, rn);
       r0 = rn[0], r1 = rn[1], r2 = rn[2];
@@ -1318,6 +1400,11 @@ __global__ void MAS_APPLY_BOUNDS(TI) k_level0_apply(ApplyArgs a, const Tv* __res
       domain_apply16<TI>(reinterpret_cast<const TI*>(slot), slot + kRecBytes16, sc, lane, x, y);
     } else {
       domain_apply(reinterpret_cast<const float*>(a.inv) + (size_t)g * kInvElems, lane, x, y);
+    }
+    if (!level0) {
+      a.coarse_z[row3] = y[0], a.coarse_z[row3 + 1] = y[1], a.coarse_z[row3 + 2] = y[2];
+      dot += (Tacc)r0 * (Tacc)y[0] + (Tacc)r1 * (Tacc)y[1] + (Tacc)r2 * (Tacc)y[2];
+      continue;
     }
     float cc[3];
     const bool real = coarse_add ? coarse_correction(a, slot, cc) : a.pmr[slot] >= 0;
@@ -1360,15 +1447,15 @@ __global__ void MAS_APPLY_BOUNDS(TI) k_level0_apply(ApplyArgs a, const Tv* __res
 // passes of the factored form read global memory once.  kBuf = 2 overlaps a
 // warp's next copy with its arithmetic; kBuf = 1 halves the shared memory per
 // warp and fits more warps per SM.  Level 0 reads r / writes z (plus the
-// coarse correction and r.z); coarse levels read and write the coarse R/Z
-// arrays.  Every wait is bounded; on expiry the warp drains its copies,
+// coarse correction and r.z); domains of level 1 (kLevel1, see
+// takes_level1) read and write the coarse R/Z arrays.  Every wait is bounded; on expiry the warp drains its copies,
 // records the error and the whole CTA leaves.
 constexpr int kApplyWarps = 4;
 
-template <typename TI, typename Tv, typename Tacc, bool kLevel0, int kBuf, bool kFused>
+template <typename TI, typename Tv, typename Tacc, int kBuf, bool kFused, bool kLevel1>
 __global__ void __launch_bounds__(kApplyWarps * 32, kBuf == 1 ? 4 : 2)
     k_apply_tma(ApplyArgs a, const Tv* __restrict__ r, Tv* z, Tacc* partial, int part_base, int total_parts, int mode,
-                PcgScalars* s, int g_begin, int g_end, int* err, int coarse_add, int pair, FusedArgs fa,
+                PcgScalars* s, int g_end, int* err, int coarse_add, int pair, FusedArgs fa,
                 double* partial_rr)
 {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -1388,7 +1475,7 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kBuf == 1 ? 4 : 2)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 #pragma unroll
     for (int j = 0; j < kBuf; ++j) {
-      const int gj = g_begin + gw + j * warps_total;
+      const int gj = gw + j * warps_total;
       if (gj < g_end) {
         mbar_expect_tx(&bar[lw][j], kBytes);
         tma_bulk_g2s(buf + j * kBytes, inv + (size_t)gj * inv_elems<TI>(), kBytes, &bar[lw][j]);
@@ -1405,7 +1492,7 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kBuf == 1 ? 4 : 2)
   if constexpr (kFused) fs = fused_scalars(s);
   int i = 0;
   bool ok = true;
-  for (int g = g_begin + gw; g < g_end; g += warps_total, ++i) {
+  for (int g = gw; g < g_end; g += warps_total, ++i) {
     const int st = kBuf == 1 ? 0 : (i & 1);
     // loads that do not depend on the record go out before its wait
     const float* scg = a.scale + (size_t)g * 96 + 3 * lane;
@@ -1413,7 +1500,8 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kBuf == 1 ? 4 : 2)
     float x[3], y[3];
     Tv rv[3];
     size_t base;
-    if (kLevel0) {
+    const bool level0 = !kLevel1 || g < a.lv.dom_begin[1];
+    if (level0) {
       base = 3 * (size_t)(a.fem_off + kBank * g + lane);
       if constexpr (kFused) {
         float rn[3];
@@ -1435,9 +1523,11 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kBuf == 1 ? 4 : 2)
       x[0] = a.coarse_r[base];
       x[1] = a.coarse_r[base + 1];
       x[2] = a.coarse_r[base + 2];
-      rv[0] = rv[1] = rv[2] = Tv(0);
+      rv[0] = x[0];
+      rv[1] = x[1];
+      rv[2] = x[2];
     }
-    const bool padded = kLevel0 && !coarse_add && a.pmr[kBank * g + lane] < 0;
+    const bool padded = level0 && !coarse_add && a.pmr[kBank * g + lane] < 0;
     const bool w = mbar_wait(&bar[lw][st], ph[st]);
     if (w) ph[st] ^= 1u;
     if (!__all_sync(kFull, w)) {
@@ -1453,7 +1543,7 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kBuf == 1 ? 4 : 2)
       mbar_expect_tx(&bar[lw][st], kBytes);
       tma_bulk_g2s(buf + st * kBytes, inv + (size_t)gn * inv_elems<TI>(), kBytes, &bar[lw][st]);
     }
-    if (kLevel0) {
+    if (level0) {
       const int slot = kBank * g + lane;
       float cc[3];
       const bool real = coarse_add ? coarse_correction(a, slot, cc) : !padded;
@@ -1471,9 +1561,11 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kBuf == 1 ? 4 : 2)
         dot += (Tacc)rv[q] * (Tacc)zv;
       }
     } else {
-      a.coarse_z[base] = y[0];
-      a.coarse_z[base + 1] = y[1];
-      a.coarse_z[base + 2] = y[2];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        a.coarse_z[base + q] = y[q];
+        dot += (Tacc)rv[q] * (Tacc)y[q];
+      }
     }
   }
   pdl_trigger();
@@ -1482,14 +1574,14 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kBuf == 1 ? 4 : 2)
     atomicExch(err, 1);
 #pragma unroll
     for (int j = 0; j < kBuf; ++j) {
-      const int gj = g_begin + gw + (i + j) * warps_total;
+      const int gj = gw + (i + j) * warps_total;
       const int sj = kBuf == 1 ? 0 : ((i + j) & 1);
       if (gj < g_end) mbar_wait(&bar[lw][sj], ph[sj]);
     }
     if (s) s->status = MASPCG_SOLVE_NONFINITE;
   }
   if (__syncthreads_or(!ok)) return;  // the whole CTA leaves together
-  if (kFused && kLevel0 && fa.update) {
+  if (kFused && fa.update) {
     // r.r of the updated residual first: its last block stores it before its
     // arrival on the r.z ticket, so the r.z completion below sees it
     double rt = 0.0;
@@ -1498,7 +1590,7 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kBuf == 1 ? 4 : 2)
         threadIdx.x == 0)
       s->rr = rt;
   }
-  if (kLevel0 && partial) {
+  if (partial) {
     Tacc total = 0;
     if (grid_finish<Tacc, kApplyWarps * 32>(dot, partial, part_base + blockIdx.x, total_parts, &s->tickets[kTicketRz],
                                             gridDim.x, total) &&
@@ -1512,10 +1604,6 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kBuf == 1 ? 4 : 2)
 }
 
 void launch_factor(maspcg_handle* h, double* assembled_out);
-namespace {
-ApplyArgs make_apply_args(maspcg_handle* h);
-}
-
 void build_mas_domains(maspcg_handle* h, double* assembled_out)
 {
   cudaStream_t st = h->stream;
@@ -1552,32 +1640,30 @@ void build_mas_domains(maspcg_handle* h, double* assembled_out)
   if (storage != MASPCG_INV_FP32) h->inv_scale.resize((size_t)lv.domains * 96);
   MCK(cudaMemsetAsync(h->failed.get() + 3, 0, sizeof(int), st));
   launch_factor(h, assembled_out);
+  // children of the coarse nodes and spans below the coarse domains (k_coarse_levels)
+  const int coarse_domains = lv.domains - lv.dom_begin[1];
+  size_t below = 0;
+  for (int l = 2; l < lv.levelnum && h->bank == 32; ++l) {
+    h->child_bank[l].resize((size_t)lv.count[l]);
+    h->child_mask[l].resize((size_t)lv.count[l]);
+    k_children<32><<<ceil_div(lv.count[l - 1], kTpb), kTpb, 0, st>>>(h->going_next.get(), lv.begin[l - 1], lv.count[l - 1],
+                                                          lv.begin[l], h->child_bank[l].get(),
+                                                          h->child_mask[l].get());
+    MLAUNCHED(h);
+    below += coarse_scratch(lv, l);
+  }
+  h->coarse_below.resize(std::max<size_t>(below, 1), 4);
+  h->coarse_span.resize((size_t)std::max(coarse_domains, 1) * kMaxLevels);
+  if (coarse_domains > 0 && h->bank == 32) {
+    k_coarse_spans<32><<<ceil_div(coarse_domains, 64), 64, 0, st>>>(
+        coarse_levels_args(h));
+    MLAUNCHED(h);
+  }
   // coarse work vectors (padding entries stay zero)
   const size_t coarse = (size_t)(lv.total_clusters - c0) * 3;
   h->coarse_r.resize(coarse > 0 ? coarse : 3);
   h->coarse_z.resize(coarse > 0 ? coarse : 3);
-  if (h->bank == 16) {
-    h->chain_dot.resize((size_t)mas16_coarse_grid(h));  // k16_apply_coarse's R.Z partials
-    MCK(cudaMemsetAsync(h->coarse_r.get(), 0, h->coarse_r.bytes(), st));
-    MCK(cudaMemsetAsync(h->coarse_z.get(), 0, h->coarse_z.bytes(), st));
-    int f = 0;
-    MCK(cudaMemcpyAsync(&f, h->failed.get() + 3, sizeof(int), cudaMemcpyDeviceToHost, st));
-    MCK(cudaStreamSynchronize(st));
-    h->failed_domains = f;
-    return;
-  }
-  const int coarse_domains = lv.domains - lv.dom_begin[1];
-  h->chain_count.resize((size_t)std::max(coarse_domains, 1));
-  h->chain_target.resize((size_t)std::max(coarse_domains, 1));
-  h->chain_dot.resize((size_t)std::max(coarse_domains, 1));
-  MCK(cudaMemsetAsync(h->chain_count.get(), 0, h->chain_count.bytes(), st));
-  MCK(cudaMemsetAsync(h->chain_target.get(), 0, h->chain_target.bytes(), st));
-  if (lv.levelnum > 1) {
-    const ApplyArgs aa = make_apply_args(h);
-    const long long units = (c0 / kBank + kChainUnitBanks - 1) / kChainUnitBanks + coarse_domains;
-    k_chain_targets<<<ceil_div(units * 32, kTpb), kTpb, 0, st>>>(aa, h->chain_target.get());
-    MLAUNCHED(h);
-  }
+  h->chain_dot.resize((size_t)std::max(coarse_domains, 1));  // >= CTAs of k16_apply_coarse
   MCK(cudaMemsetAsync(h->coarse_r.get(), 0, h->coarse_r.bytes(), st));
   MCK(cudaMemsetAsync(h->coarse_z.get(), 0, h->coarse_z.bytes(), st));
   int f = 0;
@@ -1732,10 +1818,6 @@ ApplyArgs make_apply_args(maspcg_handle* h)
   a.coarse_z = h->coarse_z.get();
   for (int l = 1; l < h->lv.levelnum && l < kMaxLevels; ++l) a.cmap[l] = h->cmap[l].get();
   a.pmr = h->pmr.get();
-  a.chain_count = h->chain_count.get();
-  a.chain_target = h->chain_target.get();
-  a.chain_dot = h->chain_dot.get();
-  a.err = h->failed.get() + 4;
   a.inv = h->inv.get();
   a.scale = h->cfg.inverse_storage == MASPCG_INV_FP32 ? nullptr : h->inv_scale.get();
   a.fem_off = h->fem_off;
@@ -1747,20 +1829,20 @@ ApplyArgs make_apply_args(maspcg_handle* h)
 // Level-0 domain apply variants (the solve uses h->apply_variant).
 enum ApplyVariant { kApplyDirect = 0, kApplyStaged2 = 1, kApplyStaged1 = 2 };
 
-template <typename TI, typename Tv, typename Tacc, bool kLevel0, int kBuf, bool kFused = false>
+template <typename TI, typename Tv, typename Tacc, int kBuf, bool kFused, bool kLevel1>
 void launch_apply_tma(maspcg_handle* h, const ApplyArgs& a, const Tv* r, Tv* z, Tacc* partial, int part_base,
-                      int total_parts, int mode, PcgScalars* s, int g_begin, int g_end, int grid, int coarse_add,
-                      int pair, const FusedArgs& fa = FusedArgs{}, double* partial_rr = nullptr)
+                      int total_parts, int mode, PcgScalars* s, int g_end, int grid, int coarse_add, int pair,
+                      const FusedArgs& fa, double* partial_rr)
 {
   constexpr int bytes = kApplyWarps * (kBuf * kRecBytes16 + kApplyScratch);
-  auto kern = k_apply_tma<TI, Tv, Tacc, kLevel0, kBuf, kFused>;
+  auto kern = k_apply_tma<TI, Tv, Tacc, kBuf, kFused, kLevel1>;
   static bool configured = false;
   if (!configured) {
     MCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     configured = true;
   }
   launch_pdl(h, kern, dim3(grid), dim3(kApplyWarps * 32), bytes, a, r, z, partial, part_base, total_parts, mode, s,
-             g_begin, g_end, h->failed.get() + 4, coarse_add, pair, fa, partial_rr);
+             g_end, h->failed.get() + 4, coarse_add, pair, fa, partial_rr);
 }
 
 // CTAs of a staged apply over `domains` domains: one wave of resident CTAs.
@@ -1769,11 +1851,12 @@ inline int staged_grid(const maspcg_handle* h, int domains, int kbuf)
   return std::max(1, std::min(ceil_div(domains, kApplyWarps), (kbuf == 1 ? 4 : 2) * h->sm_count));
 }
 
-// CTAs of the level-0 apply in a variant.  The r.z partial sums occupy one
-// slot per CTA, so the PCG engine sizes its reduction with this same count.
-inline int level0_grid(const maspcg_handle* h, int variant)
+// CTAs of the level-0 apply in a variant (level1: level 1's domains with it).
+// The r.z partial sums occupy one slot per CTA, so the PCG engine sizes its
+// reduction with this same count.
+inline int level0_grid(const maspcg_handle* h, int variant, bool level1)
 {
-  const int d0 = h->lv.dom_begin[1];
+  const int d0 = h->lv.dom_begin[level1 ? 2 : 1];
   if (h->cfg.inverse_storage == MASPCG_INV_FP32) variant = kApplyDirect;
   switch (variant) {
     case kApplyStaged2: return staged_grid(h, d0, 2);
@@ -1787,46 +1870,64 @@ inline int level0_grid(const maspcg_handle* h, int variant)
 // Level-0 apply (with r.z) in the given variant; coarse_add: z includes the
 // coarse correction (else the p update adds it); pair: r.z is completed
 // together with the concurrently running coarse levels.
-template <typename TI, typename Tv, typename Tacc, bool kFused = false>
+template <typename TI, typename Tv, typename Tacc, bool kFused = false, bool kLevel1 = false>
 void level0_apply(maspcg_handle* h, const ApplyArgs& a, int variant, const Tv* r, Tv* z, Tacc* partial, int part_base,
                   int total_parts, int mode, PcgScalars* s, int grid0, int coarse_add = 1, int pair = 0,
                   const FusedArgs& fa = FusedArgs{}, double* partial_rr = nullptr)
 {
-  const int d0 = h->lv.dom_begin[1];
+  const int g_end = h->lv.dom_begin[kLevel1 ? 2 : 1];
   if (std::is_same<TI, float>::value) variant = kApplyDirect;
-  // grid0 == level0_grid(h, variant): every CTA owns one r.z slot
+  // grid0: at least level0_grid(h, variant, kLevel1), every CTA owns one r.z slot
   switch (variant) {
     case kApplyStaged2:
       if constexpr (sizeof(TI) == 2)
-        launch_apply_tma<TI, Tv, Tacc, true, 2, kFused>(h, a, r, z, partial, part_base, total_parts, mode, s, 0, d0,
-                                                        grid0, coarse_add, pair, fa, partial_rr);
+        launch_apply_tma<TI, Tv, Tacc, 2, kFused, kLevel1>(h, a, r, z, partial, part_base, total_parts, mode, s, g_end, grid0,
+                                                  coarse_add, pair, fa, partial_rr);
       break;
     case kApplyStaged1:
       if constexpr (sizeof(TI) == 2)
-        launch_apply_tma<TI, Tv, Tacc, true, 1, kFused>(h, a, r, z, partial, part_base, total_parts, mode, s, 0, d0,
-                                                        grid0, coarse_add, pair, fa, partial_rr);
+        launch_apply_tma<TI, Tv, Tacc, 1, kFused, kLevel1>(h, a, r, z, partial, part_base, total_parts, mode, s, g_end, grid0,
+                                                  coarse_add, pair, fa, partial_rr);
       break;
 
     default:
-      launch_pdl(h, k_level0_apply<TI, Tv, Tacc, kFused>, dim3(grid0), dim3(kApplyTpb),
+      launch_pdl(h, k_level0_apply<TI, Tv, Tacc, kFused, kLevel1>, dim3(grid0), dim3(kApplyTpb),
                  sizeof(TI) == 2 ? kDirectSmem16 : 0, a, r, z, partial, part_base, total_parts, mode, s, coarse_add,
                  pair, fa, partial_rr);
       break;
   }
 }
 
-template <typename TI, typename Tv, bool kFused = false>
-void launch_chain(maspcg_handle* h, cudaStream_t st, const ApplyArgs& a, const Tv* r, PcgScalars* s, int mode, int pair,
-                  const FusedArgs& fa = FusedArgs{})
+// The coarse levels on `st`.  fa set: the residual is the fused x / r
+// update's; else restricted says that the kernel in front summed level 1's R.
+template <typename TI, typename Tv, int kB, bool kFused = false>
+void launch_coarse(maspcg_handle* h, cudaStream_t st, const ApplyArgs& a, const Tv* r, PcgScalars* s, int mode,
+                   int pair, bool restricted, const FusedArgs& fa = FusedArgs{}, int from_level = 1)
 {
-  constexpr int bytes = chain_smem_bytes<TI>();
-  auto kern = k_coarse_chain<TI, Tv, kFused>;
+  if (kFused || !restricted)
+    launch_pdl_on(h, st, k_restrict1<Tv, kB, kFused>, dim3(ceil_div(h->c0, kTpb)), dim3(kTpb), 0, a, r, s, fa);
+  if (from_level >= a.lv.levelnum) return;
+  constexpr int bytes = (kCoarseStage + 2 * 3 * kCoarseOnChip) * sizeof(float);
   static bool configured = false;
-  if (!configured && bytes > 48 * 1024)
-    MCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  if (!configured) MCK(cudaFuncSetAttribute(k_coarse_levels<TI, kB>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   configured = true;
-  launch_pdl_on(h, st, kern, dim3(ceil_div(h->c0 / kBank, kChainUnitBanks)), dim3(kChainWarps * 32), bytes, a, r, s,
-                mode, pair, fa);
+  launch_pdl_on(h, st, k_coarse_levels<TI, kB>, dim3(a.lv.domains - a.lv.dom_begin[from_level]),
+                dim3(coarse_threads<TI, kB>()), bytes, coarse_levels_args(h), s, mode, pair, h->chain_dot.get());
+}
+
+// Whether the overlapped apply takes level 1's domains into the level-0 kernel:
+// their R is there before it starts, they are the same work, and there are 1/32
+// as many.  Beside it as CTAs of k_coarse_levels they hold the registers of most
+// SMs while its own CTAs wait: 91.6 us per iteration at 262,144 rows, 86.4 this
+// way.  Where the level-0 domains are one round of resident warps no CTA waits
+// and the two ways are equal (28.9 us at 8,000 rows; 44.9 beside it and 45.3 this
+// way at 64,000).  Not where r.z is summed in FP32: the coarse share of it is an
+// FP64 sum.
+template <typename Tv, typename Tacc>
+bool takes_level1(const maspcg_handle* h)
+{
+  return sizeof(Tv) == 4 && sizeof(Tacc) == 8 && h->lv.levelnum > 1 &&
+         h->lv.dom_begin[2] > 4 * kApplyWarps * h->sm_count;
 }
 
 // The MAS apply.  Sequential form: the coarse levels, then the level-0 apply
@@ -1835,7 +1936,7 @@ void launch_chain(maspcg_handle* h, cudaStream_t st, const ApplyArgs& a, const T
 // complete r.z together, and the next p update adds the coarse correction.
 template <typename TI, typename Tv, typename Tacc>
 void mas_apply_t(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, int part_base, int total_parts, int mode,
-                 int grid0, PcgScalars* s, bool overlap)
+                 int grid0, PcgScalars* s, bool overlap, bool restricted)
 {
   ApplyArgs a = make_apply_args(h);
   const LevelInfo& lv = h->lv;
@@ -1845,15 +1946,32 @@ void mas_apply_t(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, int part_b
     return;
   }
   if (!overlap || !s) {
-    launch_chain<TI, Tv>(h, h->stream, a, r, s, mode, 0);
+    launch_coarse<TI, Tv, kBank>(h, h->stream, a, r, s, mode, 0, restricted);
     level0_apply<TI, Tv, Tacc>(h, a, variant, r, z, partial, part_base, total_parts, mode, s, grid0);
+    return;
+  }
+  const bool level1 = takes_level1<Tv, Tacc>(h);
+  const auto level0 = [&](int pair) {
+    if constexpr (sizeof(Tv) == 4 && sizeof(Tacc) == 8) {
+      if (level1) {
+        level0_apply<TI, Tv, Tacc, false, true>(h, a, variant, r, z, partial, part_base, total_parts, mode, s, grid0, 0,
+                                                pair);
+        return;
+      }
+    }
+    level0_apply<TI, Tv, Tacc>(h, a, variant, r, z, partial, part_base, total_parts, mode, s, grid0, 0, pair);
+  };
+  if (level1 && !restricted)
+    launch_pdl(h, k_restrict1<Tv, kBank, false>, dim3(ceil_div(h->c0, kTpb)), dim3(kTpb), 0, a, r, s, FusedArgs{});
+  if (level1 && lv.levelnum == 2) {
+    level0(0);
     return;
   }
   MCK(cudaEventRecord(h->ev_fork, h->stream));
   MCK(cudaStreamWaitEvent(h->side_stream, h->ev_fork, 0));
-  launch_chain<TI, Tv>(h, h->side_stream, a, r, s, mode, 1);
+  launch_coarse<TI, Tv, kBank>(h, h->side_stream, a, r, s, mode, 1, level1 || restricted, FusedArgs{}, level1 ? 2 : 1);
   MCK(cudaEventRecord(h->ev_join, h->side_stream));
-  level0_apply<TI, Tv, Tacc>(h, a, variant, r, z, partial, part_base, total_parts, mode, s, grid0, 0, 1);
+  level0(1);
   MCK(cudaStreamWaitEvent(h->stream, h->ev_join, 0));
 }
 
@@ -1877,14 +1995,14 @@ void mas_apply_fused_t(maspcg_handle* h, const FusedArgs& fa, float* z, Tacc* pa
     return;
   }
   if (!overlap) {
-    launch_chain<TI, float, true>(h, h->stream, a, nullptr, s, mode, 0, fa);
+    launch_coarse<TI, float, kBank, true>(h, h->stream, a, nullptr, s, mode, 0, false, fa);
     level0_apply<TI, float, Tacc, true>(h, a, variant, nullptr, z, partial, part_base, total_parts, mode, s, grid0, 1,
                                         0, fa, partial_rr);
     return;
   }
   MCK(cudaEventRecord(h->ev_fork, h->stream));
   MCK(cudaStreamWaitEvent(h->side_stream, h->ev_fork, 0));
-  launch_chain<TI, float, true>(h, h->side_stream, a, nullptr, s, mode, 1, fa);
+  launch_coarse<TI, float, kBank, true>(h, h->side_stream, a, nullptr, s, mode, 1, false, fa);
   MCK(cudaEventRecord(h->ev_join, h->side_stream));
   level0_apply<TI, float, Tacc, true>(h, a, variant, nullptr, z, partial, part_base, total_parts, mode, s, grid0, 0, 1,
                                       fa, partial_rr);
@@ -1900,16 +2018,18 @@ ApplyArgs mas_apply_args(maspcg_handle* h) { return make_apply_args(h); }
 // Explicit launcher used by pcg.cu.
 template <typename Tv, typename Tacc>
 void mas_apply(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, int part_base, int total_parts, int mode,
-               int grid0, PcgScalars* s, bool overlap)
+               int grid0, PcgScalars* s, bool overlap, bool restricted)
 {
   switch (h->cfg.inverse_storage) {
     case MASPCG_INV_BF16:
-      mas_apply_t<__nv_bfloat16, Tv, Tacc>(h, r, z, partial, part_base, total_parts, mode, grid0, s, overlap);
+      mas_apply_t<__nv_bfloat16, Tv, Tacc>(h, r, z, partial, part_base, total_parts, mode, grid0, s, overlap, restricted);
       break;
     case MASPCG_INV_FP16:
-      mas_apply_t<__half, Tv, Tacc>(h, r, z, partial, part_base, total_parts, mode, grid0, s, overlap);
+      mas_apply_t<__half, Tv, Tacc>(h, r, z, partial, part_base, total_parts, mode, grid0, s, overlap, restricted);
       break;
-    default: mas_apply_t<float, Tv, Tacc>(h, r, z, partial, part_base, total_parts, mode, grid0, s, overlap); break;
+    default:
+      mas_apply_t<float, Tv, Tacc>(h, r, z, partial, part_base, total_parts, mode, grid0, s, overlap, restricted);
+      break;
   }
   MCK(cudaGetLastError());
 }
@@ -1944,7 +2064,7 @@ void mas_level0_only(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, int gr
 {
   ApplyArgs a = make_apply_args(h);
   if (variant < 0) variant = h->apply_variant;
-  const int grid = level0_grid(h, variant);
+  const int grid = level0_grid(h, variant, false);
   (void)grid0;
   switch (h->cfg.inverse_storage) {
     case MASPCG_INV_BF16:
@@ -1965,13 +2085,21 @@ template void mas_level0_only<double, double>(maspcg_handle*, const double*, dou
                                               int);
 
 template void mas_apply<float, float>(maspcg_handle*, const float*, float*, float*, int, int, int, int, PcgScalars*,
-                                      bool);
+                                      bool, bool);
 template void mas_apply<float, double>(maspcg_handle*, const float*, float*, double*, int, int, int, int, PcgScalars*,
-                                       bool);
+                                       bool, bool);
 template void mas_apply<double, double>(maspcg_handle*, const double*, double*, double*, int, int, int, int,
-                                        PcgScalars*, bool);
+                                        PcgScalars*, bool, bool);
 
-int mas_level0_grid(maspcg_handle* h) { return level0_grid(h, h->apply_variant); }
+template <typename Tv, typename Tacc>
+int mas_level0_grid(maspcg_handle* h, bool overlap)
+{
+  return level0_grid(h, h->apply_variant, overlap && takes_level1<Tv, Tacc>(h));
+}
+template int mas_level0_grid<float, float>(maspcg_handle*, bool);
+template int mas_level0_grid<float, double>(maspcg_handle*, bool);
+template int mas_level0_grid<double, double>(maspcg_handle*, bool);
+
 
 // CTAs of the kernel that completes r.z (level-0 apply or prolongation).
 // CTAs of the level-0 apply, which completes r.z (or part 0 of it).  When

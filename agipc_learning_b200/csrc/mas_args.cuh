@@ -15,10 +15,6 @@ struct ApplyArgs {
   float* coarse_z;
   const void* inv;
   const float* scale;
-  int* chain_count;             // per coarse domain: arrivals so far (zero between launches)
-  const int* chain_target;      // per coarse domain: arrivals that complete it
-  double* chain_dot;            // per coarse domain: R.Z
-  int* err;
   int fem_off, c0;
   LevelInfo lv;
 };
@@ -45,6 +41,43 @@ __device__ __forceinline__ bool coarse_correction(const ApplyArgs& a, int slot, 
     }
   }
   return true;
+}
+
+// R of level 1 from one warp's 32 slots (key: the lane's level-1 node, -1 past
+// the slots and for padding, which takes no part; v: its residual row).  A
+// level-1 node's children all lie in one bank, so its sum is written, not
+// accumulated: a butterfly when every bank of the warp is one component (the
+// common case), else the component's lanes in ascending order.  Both orders are
+// fixed.
+template <int kB>
+__device__ __forceinline__ void restrict_bank(int key, float* coarse_r, const float v[3])
+{
+  const int lane = threadIdx.x & 31;
+  const unsigned grp = __match_any_sync(kFull, key >= 0 ? key : -1 - lane);
+  const unsigned bank = kB == 32 ? kFull : 0xffffu << (lane & 16);
+  float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+  if (__all_sync(kFull, grp == bank)) {
+    s0 = v[0], s1 = v[1], s2 = v[2];
+#pragma unroll
+    for (int o = kB / 2; o > 0; o >>= 1) {
+      s0 += __shfl_xor_sync(kFull, s0, o);
+      s1 += __shfl_xor_sync(kFull, s1, o);
+      s2 += __shfl_xor_sync(kFull, s2, o);
+    }
+  } else {
+    for (unsigned m = grp; __any_sync(kFull, m != 0u); m &= m - 1u) {
+      const int src = m ? __ffs(m) - 1 : lane;
+      const float a0 = __shfl_sync(kFull, v[0], src), a1 = __shfl_sync(kFull, v[1], src),
+                  a2 = __shfl_sync(kFull, v[2], src);
+      if (m) s0 += a0, s1 += a1, s2 += a2;
+    }
+  }
+  if (key >= 0 && __ffs(grp) - 1 == lane) {
+    float* d = coarse_r + 3 * (size_t)key;
+    d[0] = s0;
+    d[1] = s1;
+    d[2] = s2;
+  }
 }
 
 ApplyArgs mas_apply_args(maspcg_handle* h);

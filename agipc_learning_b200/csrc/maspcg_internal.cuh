@@ -245,8 +245,11 @@ struct maspcg_handle {
   maspcg::DBuf<int> failed;
   int failed_domains = 0;
   maspcg::DBuf<float> coarse_r, coarse_z;
-  maspcg::DBuf<int> chain_count, chain_target;  // coarse-level dataflow counters (per coarse domain)
-  maspcg::DBuf<double> chain_dot;               // per coarse domain: R.Z (r.z of the coarse levels)
+  maspcg::DBuf<int> child_bank[maspcg::kMaxLevels];       // children of the level-l nodes, l >= 2: their bank
+  maspcg::DBuf<unsigned> child_mask[maspcg::kMaxLevels];  // and lanes
+  maspcg::DBuf<int2> coarse_span;                         // per coarse domain and level: the nodes below it
+  maspcg::DBuf<float> coarse_below;  // k_coarse_levels: R below a domain where it does not fit in shared memory
+  maspcg::DBuf<double> chain_dot;  // per coarse domain: R.Z (r.z of the coarse levels)
   maspcg::DBuf<double> coarse64;
   maspcg::DBuf<double> dom64;  // 16-bit storage: assembled lower blocks between the two factor passes
   maspcg::DBuf<double> abd_inv64;

@@ -27,7 +27,7 @@ namespace maspcg {
 
 template <typename Tv, typename Tacc>
 void mas_apply(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, int part_base, int total_parts, int mode,
-               int grid0, PcgScalars* s, bool overlap);
+               int grid0, PcgScalars* s, bool overlap, bool restricted);
 
 template <typename Tv, typename Tacc>
 void mas_level0_only(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, int grid0, PcgScalars* s, int variant);
@@ -35,7 +35,8 @@ template <typename Tacc>
 void mas_apply_fused(maspcg_handle* h, const FusedArgs& fa, float* z, Tacc* partial, double* partial_rr, int part_base,
                      int total_parts, int mode, int grid0, PcgScalars* s, bool overlap);
 void launch_factor(maspcg_handle* h, double* assembled_out);
-int mas_level0_grid(maspcg_handle* h);
+template <typename Tv, typename Tacc>
+int mas_level0_grid(maspcg_handle* h, bool overlap);
 template <typename Tv, typename Tacc>
 void mas16_apply(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, int part_base, int total_parts, int mode,
                  int grid, PcgScalars* s, bool overlap);
@@ -487,6 +488,68 @@ __global__ void __launch_bounds__(kTpb) k_update_xr(Tv* x, Tv* r, const Tv* __re
     gate_check(s, (double)total, mixed);
 }
 
+// The same with R of the MAS's level 1 (the input of the coarse levels) summed
+// from the new residual on the way: a warp takes 32 slots at a time, updates
+// their 96 entries with coalesced accesses (lane, lane + 32, lane + 64), moves
+// the new r to a row per lane with shuffles and restricts it.  Rows outside the
+// MAS range follow.  Spares the coarse levels their pass over r and a launch.
+template <typename Tv, typename Tacc, int kB>
+__global__ void __launch_bounds__(kTpb) k_update_xr_restrict(ApplyArgs a, Tv* x, Tv* r, const Tv* __restrict__ p4,
+                                                             const Tv* __restrict__ ap, int nrows, int mixed,
+                                                             Tacc* partial, PcgScalars* s)
+{
+  pdl_wait();
+  if (!running(s)) return;
+  const Tv alpha = (Tv)s->alpha;
+  const int lane = threadIdx.x & 31;
+  Tacc acc = 0;
+  for (int c = (blockIdx.x * kTpb + threadIdx.x) & ~31; c < a.c0; c += gridDim.x * kTpb) {
+    const int base = 3 * (a.fem_off + c), n = 3 * min(32, a.c0 - c);
+    const int key = c + lane < a.c0 ? __ldg(a.cmap1 + c + lane) : -1;
+    Tv xx[3], rr[3], ww[3], pp[3];
+    float v[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int e = lane + 32 * k, j = base + e;
+      xx[k] = rr[k] = ww[k] = pp[k] = Tv(0);
+      if (e < n) xx[k] = x[j], rr[k] = r[j], ww[k] = ap[j], pp[k] = p4[4 * (j / 3) + j % 3];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int e = lane + 32 * k, j = base + e;
+      const Tv rn = rr[k] - alpha * ww[k];
+      v[k] = (float)rn;
+      if (e < n) {
+        x[j] = xx[k] + alpha * pp[k];
+        r[j] = rn;
+        acc += (Tacc)rn * (Tacc)rn;
+      }
+    }
+    float rv[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {  // entry 3 lane + q
+      const int e = 3 * lane + q;
+      const float t0 = __shfl_sync(kFull, v[0], e & 31), t1 = __shfl_sync(kFull, v[1], e & 31),
+                  t2 = __shfl_sync(kFull, v[2], e & 31);
+      rv[q] = e < 32 ? t0 : (e < 64 ? t1 : t2);
+    }
+    restrict_bank<kB>(key, a.coarse_r, rv);
+  }
+  const int lo = 3 * a.fem_off, skip = 3 * a.c0;
+  for (int e = blockIdx.x * kTpb + threadIdx.x; e < 3 * nrows - skip; e += gridDim.x * kTpb) {
+    const int j = e < lo ? e : e + skip;
+    x[j] = x[j] + alpha * p4[4 * (j / 3) + j % 3];
+    const Tv rn = r[j] - alpha * ap[j];
+    r[j] = rn;
+    acc += (Tacc)rn * (Tacc)rn;
+  }
+  pdl_trigger();
+  Tacc total = 0;
+  if (grid_finish<Tacc>(acc, partial, blockIdx.x, gridDim.x, &s->tickets[kTicketXr], gridDim.x, total) &&
+      threadIdx.x == 0)
+    gate_check(s, (double)total, mixed);
+}
+
 // The iteration head as one cooperative kernel (every CTA resident): the p
 // update, a grid barrier, the SpMV with p.Ap and alpha, a grid barrier, the
 // x/r update with r.r and the gate.  Saves two kernel boundaries per
@@ -843,8 +906,8 @@ struct Engine {
     gstream = h->grid_stream;
     gspmv = std::max(1, std::min(ceil_div(h->nb_int, kTpb / 16), 4 * h->sm_count));
     grows = std::max(1, std::min(ceil_div(h->nb_int, kTpb), 8 * h->sm_count));
-    gl0 = mas ? mas_level0_grid(h) : (mas16 ? mas16_grid(h) : 0);
     ovl = (mas || mas16) && h->lv.levelnum > 1 && h->overlap_coarse;
+    gl0 = mas ? mas_level0_grid<Tv, Tacc>(h, ovl) : (mas16 ? mas16_grid(h) : 0);
     const bool other = !(mas || mas16) || h->abd_bodies > 0 || h->fem_off > 0 || h->nb_int > h->fem_off + h->c0;
     gother = other ? std::max(1, std::min(ceil_div(std::max(h->nb_int, 1), kTpb), 2 * h->sm_count)) : 0;
     parts_other = gother;
@@ -890,7 +953,8 @@ struct Engine {
 
   // overlap: the coarse levels run beside the level-0 apply and z leaves the
   // coarse correction to the next p update (inside the solve only).
-  void precondition(const Tv* r, Tv* z, int mode, PcgScalars* s, bool overlap = false)
+  // restricted: level 1's R of this r is already summed (iteration_head).
+  void precondition(const Tv* r, Tv* z, int mode, PcgScalars* s, bool overlap = false, bool restricted = false)
   {
     const bool ref = h->cfg.precision == MASPCG_PREC_REFERENCE;
     if (gother) {
@@ -909,7 +973,9 @@ struct Engine {
             r, z, h->nb_int, mas_lo, mas_hi, bodies, h->abd_inv32.get(), bj ? h->diag_inv32.get() : nullptr,
             s ? partial_rz() : nullptr, 0, parts_total, any_mas ? 0 : 1, mode, s);
     }
-    if (mas) mas_apply<Tv, Tacc>(h, r, z, s ? partial_rz() : nullptr, parts_other, parts_total, mode, gl0, s, overlap);
+    if (mas)
+      mas_apply<Tv, Tacc>(h, r, z, s ? partial_rz() : nullptr, parts_other, parts_total, mode, gl0, s, overlap,
+                          restricted);
     if (mas16)
       mas16_apply<Tv, Tacc>(h, r, z, s ? partial_rz() : nullptr, parts_other, parts_total, mode, gl0, s, overlap);
     MCK(cudaGetLastError());
@@ -927,9 +993,17 @@ struct Engine {
     else
       launch_pdl(h, k_update_p<Tv, false>, dim3(grows), dim3(kTpb), 0, a, V(h->vz), V(h->vp4), h->nb_int, s);
     spmv(s);
-    launch_pdl(h, k_update_xr<Tv, Tacc>, dim3(grows), dim3(kTpb), 0, V(h->vx), V(h->vr), V(h->vp4), V(h->vap),
-               h->nb_int, mixed ? 1 : 0, partial(), s);
+    if (restricts())
+      launch_pdl(h, k_update_xr_restrict<Tv, Tacc, 32>, dim3(grows),
+                 dim3(kTpb), 0, mas_apply_args(h), V(h->vx), V(h->vr), V(h->vp4), V(h->vap), h->nb_int, mixed ? 1 : 0,
+                 partial(), s);
+    else
+      launch_pdl(h, k_update_xr<Tv, Tacc>, dim3(grows), dim3(kTpb), 0, V(h->vx), V(h->vr), V(h->vp4), V(h->vap),
+                 h->nb_int, mixed ? 1 : 0, partial(), s);
   }
+
+  // The x / r update also sums level 1's R.
+  bool restricts() const { return mas && h->lv.levelnum > 1 && !h->fused_head; }
 
   // The iteration head as one cooperative launch: one resident wave of CTAs.
   template <bool kCoarse, int kForm>
@@ -1134,8 +1208,9 @@ struct Engine {
         continue;
       }
       iteration_head(s);
-      if (mixed && it == batch - 1) true_residual(s);
-      precondition(V(h->vr), V(h->vz), 2, s, ovl);
+      const bool replace = mixed && it == batch - 1;
+      if (replace) true_residual(s);
+      precondition(V(h->vr), V(h->vz), 2, s, ovl, restricts() && !replace);
     }
   }
 
@@ -1290,8 +1365,7 @@ struct Engine {
     {
       const int terr = *h->h_err;
       MREQ(terr == 0, MASPCG_ERR_CUDA,
-           terr == 2   ? "coarse-level dataflow queue overflow in the preconditioner apply"
-           : terr == 3 ? "a grid barrier of the fused iteration kernel timed out"
+           terr == 3 ? "a grid barrier of the fused iteration kernel timed out"
                        : "a TMA mbarrier wait expired in the preconditioner apply");
     }
     float ms = 0.f;

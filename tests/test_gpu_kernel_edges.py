@@ -14,6 +14,12 @@ pytestmark = pytest.mark.gpu
 EPS32 = float(np.finfo(np.float32).eps)
 
 
+def _graph(m, s):
+    m.set_graph(s.fem_count, s.node_offset, s.neighbor_start, s.neighbor_num, s.neighbor_list, s.part_map_real,
+                s.real_map_part)
+    m.set_contacts(s.pairs)
+
+
 @pytest.mark.parametrize("nt", [1, 31, 32, 33, 129])
 def test_element_kernel_tet_counts(nt):
     """Whole and ragged warps of tets, a third of them inverted: triplets
@@ -106,6 +112,45 @@ def test_iteration_product_row_lengths(precision, matrix):
     ref = oracle.sym_spmv(1.0, A, rows, cols, xx)
     mag = oracle.sym_spmv(1.0, np.abs(A), rows, cols, np.abs(xx))
     assert np.all(np.abs(y - ref) <= eps * mag)
+
+
+def _islands(n, edge):
+    """A box mesh with only every other edge of its neighbour graph kept, so
+    that banks fall into many components at every level."""
+    s = synth.cube_system(n, E=1e5, seed=7)
+    rng = np.random.default_rng(edge)
+    keep = rng.random(s.nb) < 0.5
+    start, num, lst = s.neighbor_start, s.neighbor_num, s.neighbor_list
+    lists = [[u for u in lst[start[v]:start[v] + num[v]] if keep[u] and keep[v]] for v in range(s.nb)]
+    s.neighbor_num = np.array([len(q) for q in lists], np.uint32)
+    s.neighbor_start = np.concatenate([[0], np.cumsum(s.neighbor_num)[:-1]]).astype(np.uint32)
+    s.neighbor_list = np.array([u for q in lists for u in q], np.uint32)
+    return s
+
+
+@pytest.mark.parametrize("precision,inverse", [("reference", "fp32"), ("mixed", "bf16")])
+@pytest.mark.parametrize("n", [3, 9, 20])
+def test_apply_on_fragmented_hierarchies(n, precision, inverse):
+    """Banks of many components (whole levels of short child lists, more nodes
+    on a level than a CTA keeps on chip at n = 20) against the oracle's apply
+    with the GPU's own inverses: 1e-5, the bound of the FP32 sums."""
+    s = _islands(n, n)
+    o = oracle.Mas32.from_system(s)
+    o.reorder(s.pairs)
+    o.prepare_hessian(s.vals, s.rows, s.cols, np.arange(len(s.rows), dtype=np.uint32), 0)
+    with MasPcg(precision=precision, inverse=inverse) as m:
+        _graph(m, s)
+        m.set_matrix(s.vals, s.rows, s.cols, s.nb)
+        m.build()
+        g64, z = m.domain_matrices(), m.apply_preconditioner(s.b)
+        o64, _ = o.domains()
+        bound = oracle.Mas32.from_system(s)
+        bound.reorder(s.pairs)
+        bound.prepare_hessian(np.abs(s.vals), s.rows, s.cols, np.arange(len(s.rows), dtype=np.uint32), 0)
+        assert np.all(np.abs(g64 - o64) <= 1e-13 * bound.domains()[0] + 1e-300)
+        o.set_inverses(m.domain_inverses())
+    zo = o.precondition(s.b)
+    assert np.linalg.norm(z - zo) <= 1e-5 * np.linalg.norm(zo)
 
 
 @pytest.mark.parametrize("n", [1, 33, 2049])
