@@ -590,7 +590,7 @@ MASPCG_API maspcg_status maspcg_build_preconditioner(maspcg_handle* h)
     MREQ(h->has_matrix, MASPCG_ERR_NOT_READY, "set_matrix_bcoo first");
     if (h->mas_layout) {
       maspcg::build_hierarchy(h);
-      maspcg::build_mas_domains(h, nullptr);
+      maspcg::build_mas_domains(h);
     }
     maspcg::build_block_jacobi(h);
     MCK(cudaStreamSynchronize(h->stream));
@@ -605,7 +605,7 @@ MASPCG_API maspcg_status maspcg_refresh_matrix_values(maspcg_handle* h, const do
     MREQ(values9 != nullptr, MASPCG_ERR_INVALID_ARGUMENT, "null values");
     const double* v = device_in(h, values9, (size_t)9 * h->n_in, h->in_vals);
     maspcg::refresh_internal_values(h, v);
-    if (h->mas_layout) maspcg::build_mas_domains(h, nullptr);
+    if (h->mas_layout) maspcg::build_mas_domains(h);
     maspcg::build_block_jacobi(h);
     MCK(cudaStreamSynchronize(h->stream));
   });
@@ -627,7 +627,7 @@ MASPCG_API maspcg_status maspcg_refresh_matrix_values_indexed(maspcg_handle* h, 
     maspcg::gather_triplets(h, h->n_in, id, nullptr, nullptr, sv, source_count, 0, nullptr, nullptr,
                             h->in_vals.get());
     maspcg::refresh_internal_values(h, h->in_vals.get());
-    if (h->mas_layout) maspcg::build_mas_domains(h, nullptr);
+    if (h->mas_layout) maspcg::build_mas_domains(h);
     maspcg::build_block_jacobi(h);
     MCK(cudaStreamSynchronize(h->stream));
   });

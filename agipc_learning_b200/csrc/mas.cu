@@ -6,21 +6,16 @@
 //   * member lists: for every coarse level a stable radix sort of the fine
 //     slots by their level node, so each coarse node owns a contiguous,
 //     fixed-order list of fine rows;
-//   * one CTA per domain (all levels in one launch): warp a owns destination
-//     block-row a; it walks the fine rows of its node and every block whose
-//     column node lies in the same bank is added by the lane that owns that
-//     column -- the Galerkin sum P^T A P of prepare_hessian_bcoo_kernel and
-//     prepare_hessian_bcoo_sum_kernel (TraditionalMAS32Preconditioner.cu:
-//     2234-2464) without atomics and in a fixed order;
-//   * the 96x96 FP64 matrix stays in registers (thread (a,b) holds block
-//     (a,b)); zero diagonals become 1 (expand_symmetric_mas32 :1062-1096);
-//     FP32 storage inverts it in place by Gauss-Jordan elimination without
-//     pivoting, as __inverse6_P96x96 (:1099-1146) does, with the pivot (=
-//     the squared Cholesky diagonal) checked > 0, and stores 17 wrapped
-//     diagonals x 9 elements x 32 lanes; 16-bit storage writes the lower
-//     blocks out and k_domain_chol16 factors them (scaled BF16/FP16 tiles);
+//   * the Galerkin sums P^T A P of the coarse domains (k_coarse_assemble), as
+//     prepare_hessian_bcoo_kernel and prepare_hessian_bcoo_sum_kernel form them
+//     (TraditionalMAS32Preconditioner.cu:2234-2464); a level-0 domain is a
+//     diagonal block of the matrix itself;
+//   * one CTA per domain gathers, factors and stores it (factor.cu): zero
+//     diagonals become 1 (expand_symmetric_mas32 :1062-1096); FP32 storage
+//     keeps the inverse as 17 wrapped diagonals x 9 elements x 32 lanes, 16-bit
+//     storage the scaled Cholesky factor of the inverse (BF16/FP16 tiles);
 //   * CEMAS16: the same with 16-slot banks (48x48, FP32, 9 wrapped
-//     diagonals), with its assembly and store rules.
+//     diagonals), with its assembly rules.
 // Apply (every PCG iteration): MAS32 runs the coarse domains as one
 // kernel beside a tensor-core level-0 apply of the 16-bit records (or a warp
 // per domain on FP32 records, each stored block used for both triangles
@@ -41,16 +36,6 @@ namespace maspcg {
 namespace {
 
 constexpr int kTpb = 256;
-
-template <typename T>
-__device__ __forceinline__ T from_d(double v);
-template <>
-__device__ __forceinline__ float from_d<float>(double v) { return (float)v; }
-template <>
-__device__ __forceinline__ __nv_bfloat16 from_d<__nv_bfloat16>(double v) { return __float2bfloat16_rn((float)v); }
-template <>
-__device__ __forceinline__ __half from_d<__half>(double v) { return __float2half_rn((float)v); }
-
 
 // ------------------------------------------------------------------ build --
 
@@ -194,28 +179,15 @@ __global__ void __launch_bounds__(256) k_coarse_assemble(CoarseArgs a)
   if (node >= 0) flush(node);
 }
 
-// One CTA per domain; thread (w,lane) owns block (w,lane) of the 3kB x 3kB
-// FP64 matrix (one warp per block row; for kB = 16 lanes 16..31 only help
-// stage the gathered rows).  FP32 storage: in-place Gauss-Jordan inverse,
-// symmetric layout.  16-bit storage (kB = 32): Cholesky A = L L^T,
-// W = L^-1, stored W S^-1 with column scales S, so the applied operator
-// S (W S^-1)^T (W S^-1) S stays SPD whatever the rounding.
-template <typename TI, bool kAssembled, int kB>
-__global__ void __launch_bounds__(1024, 1) k_domain_factor(FactorArgs a, int dom_offset)
+// The packed upper FP64 blocks of a domain (the matrix its stored inverse was
+// built from, before the zero-diagonal rule): one CTA per domain, one warp per
+// block row (for kB = 16 lanes 16..31 only help stage the gathered rows).
+template <int kB>
+__global__ void __launch_bounds__(32 * kB) k_domain_gather(FactorArgs a)
 {
-  __shared__ double buf[2][96];
-  __shared__ double stage[32][16 * 9];
-  __shared__ int sdest[32][16];
-  __shared__ float sscale[96];
-  __shared__ unsigned smax[96];
-  __shared__ double spiv[2][2];  // per step: 1/pivot (GJ) or {sqrt(pivot), 1/sqrt(pivot)} (Cholesky)
-  __shared__ int fail;
-
-  const int g = blockIdx.x + dom_offset;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) fail = 0;
-  if (threadIdx.x < 96) smax[threadIdx.x] = 0u;
-
+  __shared__ double stage[kB][16 * 9];
+  __shared__ int sdest[kB][16];
+  const int g = blockIdx.x, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double acc[9];
 #pragma unroll
   for (int e = 0; e < 9; ++e) acc[e] = 0.0;
@@ -230,265 +202,13 @@ __global__ void __launch_bounds__(1024, 1) k_domain_factor(FactorArgs a, int dom
 #pragma unroll
     for (int e = 0; e < 9; ++e) acc[e] = src[e];
   }
-  if (kAssembled && lane >= w && lane < kB) {
+  if (lane >= w && lane < kB) {
     double* o = a.assembled + ((size_t)g * (kB * (kB + 1) / 2) + pkb<kB>(w, lane)) * 9;
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
       for (int j = 0; j < 3; ++j) o[i + 3 * j] = acc[3 * i + j];
   }
-  if (kAssembled && a.gather_only) return;  // uniform: no barrier has run yet
-  if (lane == w) {
-    if (acc[0] == 0.0) acc[0] = 1.0;
-    if (acc[4] == 0.0) acc[4] = 1.0;
-    if (acc[8] == 0.0) acc[8] = 1.0;
-  }
-  constexpr bool kFactored = !std::is_same<TI, float>::value;
-  static_assert(kB == 32 || !kFactored, "16-slot banks store FP32 inverses");
-  TI* out = reinterpret_cast<TI*>(a.inv) + (size_t)g * (kB == 32 ? inv_elems<TI>() : kMas16InvElems);
-
-  if (!kFactored) {
-    // ---- in-place Gauss-Jordan inversion (the elimination of __inverse6_P96x96)
-    for (int q = 0; q < kB; ++q) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const int j = 3 * q + c;
-        double* pr = buf[j & 1];
-        if (w == q) {
-          pr[3 * lane + 0] = acc[3 * c + 0];
-          pr[3 * lane + 1] = acc[3 * c + 1];
-          pr[3 * lane + 2] = acc[3 * c + 2];
-          if (lane == q) {  // the pivot's owner inverts it once for the CTA
-            double pv = acc[4 * c];
-            if (!(pv > 0.0) || !isfinite(pv)) {
-              fail = 1;
-              pv = 1.0;
-            }
-            spiv[j & 1][0] = 1.0 / pv;
-          }
-        }
-        const double m0 = __shfl_sync(kFull, acc[c], q);
-        const double m1 = __shfl_sync(kFull, acc[3 + c], q);
-        const double m2 = __shfl_sync(kFull, acc[6 + c], q);
-        __syncthreads();
-        const double inv = spiv[j & 1][0];
-        const double p[3] = {pr[3 * lane], pr[3 * lane + 1], pr[3 * lane + 2]};
-        const double mm[3] = {m0, m1, m2};
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          const bool rowj = (w == q) && (i == c);
-          const double f = mm[i] * inv;
-#pragma unroll
-          for (int jj = 0; jj < 3; ++jj) {
-            const bool colj = (lane == q) && (jj == c);
-            double& x = acc[3 * i + jj];
-            if (rowj && colj)
-              x = inv;
-            else if (rowj)
-              x = p[jj] * inv;
-            else if (colj)
-              x = -f;
-            else
-              x = fma(-f, p[jj], x);
-          }
-        }
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && fail) atomicAdd(a.failed, 1);
-    const int d = (lane - w) & (kB - 1);
-    if (lane < kB && d <= kB / 2) {
-      const bool zero = (d == kB / 2) && (w >= kB / 2);
-      if (kB == 16 && d == 0) {
-        // CEMAS16 stores the diagonal blocks with their lower elements
-        // taken from the upper ones (MASPreconditioner.cu:705-711)
-        acc[3] = acc[1];
-        acc[6] = acc[2];
-        acc[7] = acc[5];
-      }
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) out[(d * 9 + 3 * i + j) * kB + w] = from_d<TI>(zero ? 0.0 : acc[3 * i + j]);
-    }
-    return;
-  }
-  if constexpr (kFactored) {
-    // 16-bit storage: the lower blocks go to dom64 for k_domain_chol16
-    if (lane <= w) {
-      double* o = a.dom64 + ((size_t)g * kPacked + w * (w + 1) / 2 + lane) * 9;
-#pragma unroll
-      for (int e = 0; e < 9; ++e) o[e] = acc[e];
-    }
-  }
-}
-
-// 16-bit storage, second pass: the Cholesky factor of one domain from its
-// lower FP64 blocks (dom64, written by k_domain_factor), then W = L^-1 and
-// the scaled tile store.  Thread t < 528 owns lower block (w, lane),
-// t = w(w+1)/2 + lane; only the lower triangle takes part, so two CTAs fit
-// on an SM and hide each other's step latency.  The steps talk through
-// shared memory only, so the thread layout is free.
-constexpr int kCholThreads = 544;  // 528 lower blocks in 17 warps
-template <typename TI>
-__global__ void __launch_bounds__(kCholThreads, 2) k_domain_chol16(FactorArgs a, int dom_offset)
-{
-  __shared__ double dinv[kBank][9];      // L_qq^-1 (lower, row-major), kept for W below
-  __shared__ double panel[2][kBank][9];  // L_wq
-  __shared__ double wrow[2][kBank][9];   // W_ql
-  __shared__ float sscale[96];
-  __shared__ unsigned smax[96];
-  __shared__ int fail;
-  const int g = blockIdx.x + dom_offset;
-  const bool act = threadIdx.x < kPacked;
-  int w = -1, lane = -1;
-  if (act) {
-    const int t = threadIdx.x;
-    w = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
-    while (w * (w + 1) / 2 > t) --w;
-    while ((w + 1) * (w + 2) / 2 <= t) ++w;
-    lane = t - w * (w + 1) / 2;
-  }
-  if (threadIdx.x == 0) fail = 0;
-  if (threadIdx.x < 96) smax[threadIdx.x] = 0u;
-  double acc[9];
-  if (act) {
-    const double* src = a.dom64 + ((size_t)g * kPacked + threadIdx.x) * 9;
-#pragma unroll
-    for (int e = 0; e < 9; ++e) acc[e] = src[e];
-  } else {
-#pragma unroll
-    for (int e = 0; e < 9; ++e) acc[e] = 0.0;
-  }
-  __syncthreads();
-  // ---- blocked Cholesky, right-looking over the 32 block columns: thread
-  // (q,q) factors its 3x3 diagonal block and inverts the factor, the block
-  // column below it is solved against that factor, then the trailing lower
-  // blocks take the rank-3 update.  Lower blocks (w >= lane) hold L after.
-  for (int q = 0; q < kBank; ++q) {
-    const int b = q & 1;
-    if (w == q && lane == q) {
-      double p0 = acc[0];
-      if (!(p0 > 0.0) || !isfinite(p0)) fail = 1, p0 = 1.0;
-      const double l00 = sqrt(p0), i00 = 1.0 / l00;
-      const double l10 = acc[3] * i00, l20 = acc[6] * i00;
-      double p1 = acc[4] - l10 * l10;
-      if (!(p1 > 0.0) || !isfinite(p1)) fail = 1, p1 = 1.0;
-      const double l11 = sqrt(p1), i11 = 1.0 / l11;
-      const double l21 = (acc[7] - l20 * l10) * i11;
-      double p2 = acc[8] - l20 * l20 - l21 * l21;
-      if (!(p2 > 0.0) || !isfinite(p2)) fail = 1, p2 = 1.0;
-      const double l22 = sqrt(p2), i22 = 1.0 / l22;
-      const double i10 = -(l10 * i00) * i11;
-      const double i21 = -(l21 * i11) * i22;
-      const double i20 = -(l20 * i00 + l21 * i10) * i22;
-      const double L[9] = {l00, 0.0, 0.0, l10, l11, 0.0, l20, l21, l22};
-      const double I[9] = {i00, 0.0, 0.0, i10, i11, 0.0, i20, i21, i22};
-#pragma unroll
-      for (int e = 0; e < 9; ++e) {
-        acc[e] = L[e];
-        dinv[q][e] = I[e];
-      }
-    }
-    __syncthreads();
-    if (lane == q && w > q) {  // L_wq = A_wq L_qq^-T
-      double l[9];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-          l[3 * i + j] = acc[3 * i] * dinv[q][3 * j] + acc[3 * i + 1] * dinv[q][3 * j + 1] +
-                         acc[3 * i + 2] * dinv[q][3 * j + 2];
-#pragma unroll
-      for (int e = 0; e < 9; ++e) {
-        acc[e] = l[e];
-        panel[b][w][e] = l[e];
-      }
-    }
-    __syncthreads();
-    if (w > q && lane > q && lane <= w) {  // A_wl -= L_wq L_lq^T
-      const double* pw = panel[b][w];
-      const double* pl = panel[b][lane];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-          acc[3 * i + j] -= pw[3 * i] * pl[3 * j] + pw[3 * i + 1] * pl[3 * j + 1] + pw[3 * i + 2] * pl[3 * j + 2];
-    }
-  }
-  // ---- W = L^-1 by blocked forward substitution on the identity: row
-  // block q of W is L_qq^-1 times the current right-hand side, which is then
-  // eliminated from the rows below.
-  double xr[9];
-#pragma unroll
-  for (int e = 0; e < 9; ++e) xr[e] = (w == lane && (e % 4) == 0) ? 1.0 : 0.0;
-  for (int q = 0; q < kBank; ++q) {
-    const int b = q & 1;
-    if (lane == q && w > q) {
-#pragma unroll
-      for (int e = 0; e < 9; ++e) panel[b][w][e] = acc[e];  // L_wq
-    }
-    if (w == q && lane <= q) {  // W_ql = L_qq^-1 X_ql
-      double y[9];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-          y[3 * i + j] = dinv[q][3 * i] * xr[j] + dinv[q][3 * i + 1] * xr[3 + j] + dinv[q][3 * i + 2] * xr[6 + j];
-#pragma unroll
-      for (int e = 0; e < 9; ++e) {
-        xr[e] = y[e];
-        wrow[b][lane][e] = y[e];
-      }
-    }
-    __syncthreads();
-    if (w > q && lane <= q) {  // X_wl -= L_wq W_ql
-      const double* lw = panel[b][w];
-      const double* wl = wrow[b][lane];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-          xr[3 * i + j] -= lw[3 * i] * wl[j] + lw[3 * i + 1] * wl[3 + j] + lw[3 * i + 2] * wl[6 + j];
-    }
-  }
-  __syncthreads();
-  // ---- column scales and factored store (lower blocks only)
-  if (act) {
-#pragma unroll
-    for (int jj = 0; jj < 3; ++jj) {
-      const float m = (float)fmax(fmax(fabs(xr[jj]), fabs(xr[3 + jj])), fabs(xr[6 + jj]));
-      atomicMax(smax + 3 * lane + jj, __float_as_uint(m));
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < 96) {
-    float sv = __uint_as_float(smax[threadIdx.x]);
-    if (!(sv > 0.f) || !isfinite(sv)) sv = 1.f;
-    sscale[threadIdx.x] = sv;
-    a.scale[(size_t)g * 96 + threadIdx.x] = sv;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0 && fail) atomicAdd(a.failed, 1);
-  // tile store: lower blocks, and zeros for the upper elements that fall in
-  // a diagonal tile
-  if (!act) return;
-  TI* out = reinterpret_cast<TI*>(a.inv) + (size_t)g * kInvElems16;
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int jj = 0; jj < 3; ++jj) {
-      // (an upper element outside the diagonal tiles has no slot: a 3x3
-      // diagonal block can straddle a tile boundary)
-      const int row = 3 * w + i, col = 3 * lane + jj;
-      if (row >= col)
-        out[inv16_pos(row, col)] = from_d<TI>(xr[3 * i + jj] / (double)sscale[3 * lane + jj]);
-      else if ((row >> 4) == (col >> 4))
-        out[inv16_pos(row, col)] = from_d<TI>(0.0);
-      // the mirror upper block (lane, w): its elements inside a diagonal tile are zero
-      const int mr = 3 * lane + i, mc = 3 * w + jj;
-      if (w > lane && (mr >> 4) == (mc >> 4)) out[inv16_pos(mr, mc)] = from_d<TI>(0.0);
-    }
 }
 
 // ------------------------------------------------------------------ apply --
@@ -1603,8 +1323,8 @@ __global__ void __launch_bounds__(kApplyWarps * 32, kBuf == 1 ? 4 : 2)
   }
 }
 
-void launch_factor(maspcg_handle* h, double* assembled_out);
-void build_mas_domains(maspcg_handle* h, double* assembled_out)
+void launch_factor(maspcg_handle* h);
+void build_mas_domains(maspcg_handle* h)
 {
   cudaStream_t st = h->stream;
   const LevelInfo& lv = h->lv;
@@ -1639,7 +1359,7 @@ void build_mas_domains(maspcg_handle* h, double* assembled_out)
   h->inv.resize((size_t)lv.domains * (h->bank == 16 ? kMas16InvElems : inv_elems_for(storage)) * esize, 16);
   if (storage != MASPCG_INV_FP32) h->inv_scale.resize((size_t)lv.domains * 96);
   MCK(cudaMemsetAsync(h->failed.get() + 3, 0, sizeof(int), st));
-  launch_factor(h, assembled_out);
+  launch_factor(h);
   // children of the coarse nodes and spans below the coarse domains (k_coarse_levels)
   const int coarse_domains = lv.domains - lv.dom_begin[1];
   size_t below = 0;
@@ -1672,17 +1392,33 @@ void build_mas_domains(maspcg_handle* h, double* assembled_out)
   h->failed_domains = f;
 }
 
+FactorArgs factor_args(maspcg_handle* h)
+{
+  FactorArgs fa{};
+  fa.lv = h->lv;
+  fa.pmr = h->pmr.get();
+  fa.rowptr = h->rowptr.get();
+  fa.colidx = h->colidx.get();
+  fa.val64 = h->val64.get();
+  fa.fem_off = h->fem_off;
+  fa.c0 = h->c0;
+  fa.inv = h->inv.get();
+  fa.scale = h->inv_scale.get();
+  fa.failed = h->failed.get() + 3;
+  fa.coarse64 = h->coarse64.get();
+  return fa;
+}
+
+// Coarse-level Galerkin sums, then the inverse of every domain (factor.cu).
 template <int kB>
-void launch_factor_t(maspcg_handle* h, double* assembled_out, bool gather_only = false)
+void launch_factor_t(maspcg_handle* h)
 {
   cudaStream_t st = h->stream;
   const LevelInfo& lv = h->lv;
-  const int c0 = h->c0;
   const int storage = kB == 16 ? (int)MASPCG_INV_FP32 : h->cfg.inverse_storage;
   const int d0 = lv.dom_begin[1];
   const int coarse_domains = lv.domains - d0;
-  // coarse-level Galerkin sums (kept from the build when only gathering)
-  if (!gather_only) h->coarse64.resize((size_t)std::max(coarse_domains, 1) * kB * kB * 9);
+  h->coarse64.resize((size_t)std::max(coarse_domains, 1) * kB * kB * 9);
   CoarseArgs ca{};
   ca.pmr = h->pmr.get();
   ca.prefix_orig = h->prefix_orig.get();
@@ -1702,110 +1438,54 @@ void launch_factor_t(maspcg_handle* h, double* assembled_out, bool gather_only =
   ca.colidx = h->colidx.get();
   ca.val64 = h->val64.get();
   ca.fem_off = h->fem_off;
-  ca.c0 = c0;
+  ca.c0 = h->c0;
   ca.coarse64 = h->coarse64.get();
   // The coarse sums feed only the coarse domains: with level-0 domains to
   // factor they are assembled on the side stream meanwhile, and the coarse
   // domains are factored after the join.
-  const bool split = !gather_only && items > 0 && d0 > 0 && coarse_domains > 0;
-  if (!gather_only) {
-    cudaStream_t cs = st;
-    if (split) {
-      MCK(cudaEventRecord(h->ev_fork, st));
-      MCK(cudaStreamWaitEvent(h->side_stream, h->ev_fork, 0));
-      cs = h->side_stream;
-    }
-    MCK(cudaMemsetAsync(h->coarse64.get(), 0, (size_t)coarse_domains * kB * kB * 9 * sizeof(double), cs));
-    if (items > 0) {
-      k_coarse_assemble<kB><<<ceil_div((long long)items * 32, 256), 256, 0, cs>>>(ca);
-      MLAUNCHED(h);
-    }
-    if (split) MCK(cudaEventRecord(h->ev_join, cs));
-  }
-  FactorArgs fa{};
-  fa.lv = lv;
-  for (int l = 1; l < lv.levelnum; ++l) {
-    fa.cmap[l] = h->cmap[l].get();
-    fa.perm[l] = h->perm[l].get();
-    fa.off[l] = h->off[l].get();
-  }
-  fa.pmr = h->pmr.get();
-  fa.rowptr = h->rowptr.get();
-  fa.colidx = h->colidx.get();
-  fa.val64 = h->val64.get();
-  fa.fem_off = h->fem_off;
-  fa.c0 = c0;
-  fa.inv = h->inv.get();
-  fa.scale = storage == MASPCG_INV_FP32 ? nullptr : h->inv_scale.get();
-  fa.failed = h->failed.get() + 3;
-  fa.assembled = assembled_out;
-  fa.coarse64 = h->coarse64.get();
-  fa.gather_only = gather_only ? 1 : 0;
-  if (kB == 32 && storage != MASPCG_INV_FP32 && !gather_only) {
-    h->dom64.resize((size_t)lv.domains * kPacked * 9);
-    fa.dom64 = h->dom64.get();
-  }
-  // domains [g0, g0 + n): gather / Gauss-Jordan, then the 16-bit Cholesky
-  auto factor = [&](int g0, int n) {
-    if (n <= 0) return;
-#define MAS_FACTOR(TI, ASM) k_domain_factor<TI, ASM, kB><<<n, 32 * kB, 0, st>>>(fa, g0)
-    if constexpr (kB == 16) {
-      if (assembled_out)
-        MAS_FACTOR(float, true);
-      else
-        MAS_FACTOR(float, false);
-    } else if (assembled_out) {
-      if (storage == MASPCG_INV_FP32)
-        MAS_FACTOR(float, true);
-      else if (storage == MASPCG_INV_BF16)
-        MAS_FACTOR(__nv_bfloat16, true);
-      else
-        MAS_FACTOR(__half, true);
-    } else {
-      if (storage == MASPCG_INV_FP32)
-        MAS_FACTOR(float, false);
-      else if (storage == MASPCG_INV_BF16)
-        MAS_FACTOR(__nv_bfloat16, false);
-      else
-        MAS_FACTOR(__half, false);
-    }
-#undef MAS_FACTOR
-    MLAUNCHED(h);
-    if (gather_only) return;
-    if constexpr (kB == 32) {
-      if (storage == MASPCG_INV_BF16) {
-        k_domain_chol16<__nv_bfloat16><<<n, kCholThreads, 0, st>>>(fa, g0);
-        MLAUNCHED(h);
-      } else if (storage == MASPCG_INV_FP16) {
-        k_domain_chol16<__half><<<n, kCholThreads, 0, st>>>(fa, g0);
-        MLAUNCHED(h);
-      }
-    }
-  };
+  const bool split = items > 0 && d0 > 0 && coarse_domains > 0;
+  cudaStream_t cs = st;
   if (split) {
-    factor(0, d0);
+    MCK(cudaEventRecord(h->ev_fork, st));
+    MCK(cudaStreamWaitEvent(h->side_stream, h->ev_fork, 0));
+    cs = h->side_stream;
+  }
+  MCK(cudaMemsetAsync(h->coarse64.get(), 0, (size_t)coarse_domains * kB * kB * 9 * sizeof(double), cs));
+  if (items > 0) {
+    k_coarse_assemble<kB><<<ceil_div((long long)items * 32, 256), 256, 0, cs>>>(ca);
+    MLAUNCHED(h);
+  }
+  if (split) MCK(cudaEventRecord(h->ev_join, cs));
+  const FactorArgs fa = factor_args(h);
+  if (split) {
+    factor_domains(h, fa, 0, d0, storage);
     MCK(cudaStreamWaitEvent(st, h->ev_join, 0));
-    factor(d0, lv.domains - d0);
+    factor_domains(h, fa, d0, coarse_domains, storage);
   } else {
-    factor(0, lv.domains);
+    factor_domains(h, fa, 0, lv.domains, storage);
   }
   MCK(cudaGetLastError());
 }
 
-void launch_factor(maspcg_handle* h, double* assembled_out)
+void launch_factor(maspcg_handle* h)
 {
   if (h->bank == 16)
-    launch_factor_t<16>(h, assembled_out);
+    launch_factor_t<16>(h);
   else
-    launch_factor_t<32>(h, assembled_out);
+    launch_factor_t<32>(h);
 }
 
 void gather_mas_domains(maspcg_handle* h, double* assembled_out)
 {
+  FactorArgs fa = factor_args(h);
+  fa.assembled = assembled_out;
+  if (h->lv.domains <= 0) return;
   if (h->bank == 16)
-    launch_factor_t<16>(h, assembled_out, true);
+    k_domain_gather<16><<<h->lv.domains, 512, 0, h->stream>>>(fa);
   else
-    launch_factor_t<32>(h, assembled_out, true);
+    k_domain_gather<32><<<h->lv.domains, 1024, 0, h->stream>>>(fa);
+  MLAUNCHED(h);
+  MCK(cudaGetLastError());
 }
 
 namespace {

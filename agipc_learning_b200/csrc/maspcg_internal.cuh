@@ -170,12 +170,9 @@ struct LevelInfo {
   int domains;
 };
 
-// Pointers used by the domain factorisation kernel, one entry per level.
+// Pointers used by the domain gather and factorisation kernels.
 struct FactorArgs {
   LevelInfo lv;
-  const int* cmap[kMaxLevels];   // fine slot -> level-L local node (-1 padding); level 0 unused
-  const int* perm[kMaxLevels];   // level-L member lists (fine slots), level >= 1
-  const int* off[kMaxLevels];    // level-L member offsets [count+1], level >= 1
   const int* pmr;                // part_map_real
   const int* rowptr;
   const int* colidx;
@@ -187,8 +184,6 @@ struct FactorArgs {
   int* failed;                   // count of domains with a pivot <= 0
   double* assembled;             // optional: packed FP64 domain matrices (reference layout)
   const double* coarse64;        // coarse-level domain matrices (32x32 blocks, row-major 3x3)
-  double* dom64;                 // 16-bit storage: lower FP64 blocks per domain (kPacked x 9, row-major)
-  int gather_only;               // write `assembled` and stop: the stored inverses are left as they are
 };
 
 }  // namespace maspcg
@@ -251,7 +246,6 @@ struct maspcg_handle {
   maspcg::DBuf<float> coarse_below;  // k_coarse_levels: R below a domain where it does not fit in shared memory
   maspcg::DBuf<double> chain_dot;  // per coarse domain: R.Z (r.z of the coarse levels)
   maspcg::DBuf<double> coarse64;
-  maspcg::DBuf<double> dom64;  // 16-bit storage: assembled lower blocks between the two factor passes
   maspcg::DBuf<double> abd_inv64;
   maspcg::DBuf<float> abd_inv32;
   maspcg::DBuf<double> diag_inv64;
@@ -319,12 +313,13 @@ void permute_out(maspcg_handle* h, const double* src_int, double* dst_orig);
 void build_block_jacobi(maspcg_handle* h);
 
 // mas.cu
-void build_mas_domains(maspcg_handle* h, double* assembled_out);
+void build_mas_domains(maspcg_handle* h);
 // The packed FP64 domain matrices the stored inverses were built from: level
 // 0 gathered again (a fixed order), the coarse levels from the build's own
 // Galerkin sums; neither the sums nor the inverses are recomputed.
 void gather_mas_domains(maspcg_handle* h, double* assembled_out);
-void mas_apply_launch(maspcg_handle* h, const void* r, void* z, bool finalize_rz);
+// factor.cu: inverses of the domains [g0, g0 + n)
+void factor_domains(maspcg_handle* h, const FactorArgs& a, int g0, int n, int storage);
 void decode_inverses(maspcg_handle* h, float* out_host);
 
 // Count one launch of this library (graph captures are corrected afterwards).

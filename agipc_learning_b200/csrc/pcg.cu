@@ -34,7 +34,7 @@ void mas_level0_only(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, int gr
 template <typename Tacc>
 void mas_apply_fused(maspcg_handle* h, const FusedArgs& fa, float* z, Tacc* partial, double* partial_rr, int part_base,
                      int total_parts, int mode, int grid0, PcgScalars* s, bool overlap);
-void launch_factor(maspcg_handle* h, double* assembled_out);
+void launch_factor(maspcg_handle* h);
 template <typename Tv, typename Tacc>
 int mas_level0_grid(maspcg_handle* h, bool overlap);
 template <typename Tv, typename Tacc>
@@ -1250,7 +1250,7 @@ struct Engine {
         case 0: spmv(s); break;
         case 1: precondition(V(h->vr), V(h->vz), 0, s); break;
         case 2: mas_level0_only<Tv, Tacc>(h, V(h->vr), V(h->vz), partial_rz(), gl0, s, -1); break;
-        case 3: launch_factor(h, nullptr); break;
+        case 3: launch_factor(h); break;
         case 7: true_residual(s); break;
         default: mas_level0_only<Tv, Tacc>(h, V(h->vr), V(h->vz), partial_rz(), gl0, s, stage == 6 ? 0 : stage - 3);
       }
