@@ -247,7 +247,6 @@ struct maspcg_handle {
   maspcg::DBuf<double> chain_dot;  // per coarse domain: R.Z (r.z of the coarse levels)
   maspcg::DBuf<double> coarse64;
   maspcg::DBuf<double> abd_inv64;
-  maspcg::DBuf<float> abd_inv32;
   maspcg::DBuf<double> diag_inv64;
   maspcg::DBuf<float> diag_inv32;
 

@@ -667,34 +667,53 @@ __global__ void __launch_bounds__(kTpb) k_true_residual(const int* __restrict__ 
   }
 }
 
-// Rows outside the MAS range: affine bodies (12x12 inverse), the 3x3
+// z = P r for the affine bodies' FP64 12x12 inverses, 16 bodies per CTA and a
+// thread per row: the inverses come in coalesced and are read from shared memory
+// (rows padded to 13, no bank conflicts).  One thread per body, walking 1,152
+// bytes of its own, took 25 us for the 500 bodies of the hybrid system.
+constexpr int kBodyTpb = 192;
+template <typename Tv>
+__global__ void __launch_bounds__(kBodyTpb) k_body_apply(const Tv* __restrict__ r, Tv* z, int bodies,
+                                                        const double* __restrict__ inv, const PcgScalars* s)
+{
+  __shared__ double P[kBodyTpb][13];
+  __shared__ double in[kBodyTpb];
+  const int first = blockIdx.x * (kBodyTpb / 12), rows = 12 * min(kBodyTpb / 12, bodies - first);
+  for (int e = threadIdx.x; e < 12 * rows; e += kBodyTpb) P[e / 12][e % 12] = __ldg(inv + 144 * (size_t)first + e);
+  pdl_wait();
+  if (s && s->status != MASPCG_SOLVE_RUNNING) return;
+  const int t = threadIdx.x;
+  if (t < rows) in[t] = (double)r[12 * (size_t)first + t];
+  __syncthreads();
+  if (t >= rows) return;
+  double acc = 0.0;
+#pragma unroll
+  for (int c = 0; c < 12; ++c) acc += P[t][c] * in[t / 12 * 12 + c];
+  z[12 * (size_t)first + t] = (Tv)acc;
+}
+
+// Rows outside the MAS range: the affine bodies' share of r.z, the 3x3
 // block-Jacobi rows, identity elsewhere (global_linear_system.cu:293-306).
 // When `finalize` is set this kernel completes the r.z reduction.
 template <typename Tv, typename Tacc, typename Tinv>
 __global__ void __launch_bounds__(kTpb) k_other_apply(const Tv* __restrict__ r, Tv* z, int nb_int, int mas_lo,
-                                                       int mas_hi, int bodies, const Tinv* __restrict__ abd_inv,
-                                                       const Tinv* __restrict__ diag_inv, Tacc* partial, int part_base,
-                                                       int total_parts, int finalize, int mode, PcgScalars* s)
+                                                       int mas_hi, int bodies, const Tinv* __restrict__ diag_inv, Tacc* partial,
+                                                       int part_base, int total_parts, int finalize, int mode, PcgScalars* s)
 {
   pdl_wait();
   if (s && s->status != MASPCG_SOLVE_RUNNING) return;
   Tacc dot = 0;
   const int stride = gridDim.x * blockDim.x;
-  // bodies: one thread per body
-  for (int bdy = blockIdx.x * blockDim.x + threadIdx.x; bdy < bodies; bdy += stride) {
-    const Tinv* P = abd_inv + 144 * (size_t)bdy;
-    Tv in[12];
+  // bodies: their z comes from k_body_apply; a thread per body adds its share
+  // of r.z, the rows in order
+  if (partial)
+    for (int bdy = blockIdx.x * blockDim.x + threadIdx.x; bdy < bodies; bdy += stride) {
+      Tv in[12], out[12];
 #pragma unroll
-    for (int c = 0; c < 12; ++c) in[c] = r[12 * (size_t)bdy + c];
-#pragma unroll 1
-    for (int a = 0; a < 12; ++a) {
-      Tinv acc = 0;
+      for (int c = 0; c < 12; ++c) in[c] = r[12 * (size_t)bdy + c], out[c] = z[12 * (size_t)bdy + c];
 #pragma unroll
-      for (int c = 0; c < 12; ++c) acc += P[12 * a + c] * (Tinv)in[c];
-      z[12 * (size_t)bdy + a] = (Tv)acc;
-      dot += (Tacc)in[a] * (Tacc)(Tv)acc;
+      for (int c = 0; c < 12; ++c) dot += (Tacc)in[c] * (Tacc)out[c];
     }
-  }
   // remaining rows
   const int first = 4 * bodies;
   for (int row = first + blockIdx.x * blockDim.x + threadIdx.x; row < nb_int; row += stride) {
@@ -944,7 +963,7 @@ struct Engine {
                    mas_hi, bodies, (const double*)h->abd_inv64.get(), partial_rz(), h->partial_rr.get(), s);
       else
         launch_pdl(h, k_other_apply_fused<Tacc, float>, dim3(gother), dim3(kTpb), 0, f, Vf(h->vz), h->nb_int, mas_lo,
-                   mas_hi, bodies, (const float*)h->abd_inv32.get(), partial_rz(), h->partial_rr.get(), s);
+                   mas_hi, bodies, (const float*)nullptr, partial_rz(), h->partial_rr.get(), s);
     }
     mas_apply_fused<Tacc>(h, f, Vf(h->vz), partial_rz(), h->partial_rr.get(), parts_other, parts_total, mode, gl0, s,
                           ovl);
@@ -964,13 +983,16 @@ struct Engine {
       const int bodies = (h->cfg.preconditioner == MASPCG_PRECOND_NONE) ? 0 : h->abd_bodies;
       // affine bodies always apply their FP64 inverses: the 12x12 inverse
       // spans the same ~1e11 spread as the body's Hessian block
+      if (bodies > 0)
+        launch_pdl(h, k_body_apply<Tv>, dim3(ceil_div(bodies, kBodyTpb / 12)), dim3(kBodyTpb), 0, r, z, bodies,
+                   h->abd_inv64.get(), s);
       if (ref || bodies > 0)
         launch_pdl(h, k_other_apply<Tv, Tacc, double>, dim3(gother), dim3(kTpb), 0, 
-            r, z, h->nb_int, mas_lo, mas_hi, bodies, h->abd_inv64.get(), bj ? h->diag_inv64.get() : nullptr,
+            r, z, h->nb_int, mas_lo, mas_hi, bodies, bj ? h->diag_inv64.get() : nullptr,
             s ? partial_rz() : nullptr, 0, parts_total, any_mas ? 0 : 1, mode, s);
       else
         launch_pdl(h, k_other_apply<Tv, Tacc, float>, dim3(gother), dim3(kTpb), 0, 
-            r, z, h->nb_int, mas_lo, mas_hi, bodies, h->abd_inv32.get(), bj ? h->diag_inv32.get() : nullptr,
+            r, z, h->nb_int, mas_lo, mas_hi, bodies, bj ? h->diag_inv32.get() : nullptr,
             s ? partial_rz() : nullptr, 0, parts_total, any_mas ? 0 : 1, mode, s);
     }
     if (mas)

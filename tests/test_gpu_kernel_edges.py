@@ -178,3 +178,35 @@ def test_block_gradient_checks_every_index(n):
     g = -L[r][:, :, None] * X[c][:, None, :]
     g -= np.where((r != c)[:, None, None], X[r][:, :, None] * L[c][:, None, :], 0.0)
     assert np.allclose(out.cpu().numpy(), g.transpose(0, 2, 1).reshape(-1, 9), rtol=1e-14, atol=1e-14)
+
+
+@pytest.mark.parametrize("precision", ["reference", "mixed"])
+@pytest.mark.parametrize("bodies", [1, 3, 4, 5, 16, 17, 33])
+def test_body_inverses_and_apply(bodies, precision):
+    """12x12 bodies around a CTA's share of them (4 to invert, 16 to apply),
+    every other one needing row exchanges: each body's z against a solve, within
+    its condition number times eps (FP64; plus z's own rounding in FP32)."""
+    rng = np.random.default_rng(bodies)
+    nb, rows, cols, vals, dense = 4 * bodies + 5, [], [], [], []
+    for k in range(bodies):
+        A = rng.standard_normal((12, 12))
+        A = A + A.T + (0.0 if k % 2 else 20.0 * np.eye(12))
+        if k % 2:
+            A[0, 0] = A[3, 3] = 0.0
+        dense.append(A)
+        for i in range(4):
+            for j in range(i, 4):
+                rows.append(4 * k + i), cols.append(4 * k + j), vals.append(A[3 * i:3 * i + 3, 3 * j:3 * j + 3].T.reshape(9))
+    for i in range(4 * bodies, nb):
+        rows.append(i), cols.append(i), vals.append(2.0 * np.eye(3).reshape(9))
+    b = rng.standard_normal(3 * nb)
+    with MasPcg(preconditioner="block_jacobi", precision=precision) as m:
+        m.set_matrix(np.array(vals), np.array(rows, np.int32), np.array(cols, np.int32), nb, 4 * bodies, bodies)
+        m.build()
+        z = m.apply_preconditioner(b)
+    eps = np.finfo(np.float64).eps if precision == "reference" else EPS32
+    for k, A in enumerate(dense):
+        zk = np.linalg.solve(A, b[12 * k:12 * k + 12])
+        tol = 144 * np.finfo(np.float64).eps * np.linalg.cond(A) + 4 * eps * np.linalg.cond(A)
+        assert np.linalg.norm(z[12 * k:12 * k + 12] - zk) <= tol * np.linalg.norm(zk), k
+    assert np.allclose(z[12 * bodies:], b[12 * bodies:] / 2, rtol=1e-6)
