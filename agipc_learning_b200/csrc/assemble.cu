@@ -1,9 +1,10 @@
 // assemble.cu -- the two triplet steps in front of the solve, on the device:
 //
 // * convert_bcoo: Converter::convert (StiffGIPC/linear_system/utils/
-//   converter.cu:137-284).  Triplets keyed (row << 32) + col (packed into as
-//   few bits as the indices need: the same order) are radix-sorted (stable), runs of equal keys are found with head flags and an exclusive
-//   scan, and each run's 3x3 blocks are summed.  The reference sums a run with
+//   converter.cu:137-284).  Triplets are put in the stable order of (row, col)
+//   by row buckets (rowsort.cu), or, where a row is too long for those, by a
+//   radix sort of the key (row << 32) + col packed into as few bits as the
+//   indices need, and each run's 3x3 blocks are summed.  The reference sums a run with
 //   a warp head-segmented reduction plus FP64 atomics, whose order varies;
 //   here each element of a block is summed over its run in the stable sort
 //   order, so the result is deterministic (and equal to a sequential sum in input order within each
@@ -72,11 +73,19 @@ __global__ void k_conv_heads(const unsigned long long* __restrict__ keys, int n,
   if (i < n) heads[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1 : 0;
 }
 
-// start[u] = first sorted position of unique key u; start[count] = n
-__global__ void k_conv_starts(const int* __restrict__ heads, const int* __restrict__ pos, int n, int* start)
+// start[u] = first sorted position of unique key u; start[count] = n; its row
+// and column
+__global__ void k_conv_starts(const int* __restrict__ heads, const int* __restrict__ pos,
+                              const unsigned long long* __restrict__ keys, int n, int col_bits, int* start, int* urow,
+                              int* ucol)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && heads[i]) start[pos[i]] = i;
+  if (i < n && heads[i]) {
+    const int u = pos[i];
+    start[u] = i;
+    urow[u] = (int)(keys[i] >> col_bits);
+    ucol[u] = (int)(keys[i] & ((1ull << col_bits) - 1ull));
+  }
   if (i == n - 1) start[pos[i] + heads[i]] = n;
 }
 
@@ -86,30 +95,23 @@ __global__ void k_conv_starts(const int* __restrict__ heads, const int* __restri
 // entries are fetched four ahead of the sums.  Bound by the latency of the
 // scattered blocks.  On the 110,592-row merge the whole call went from 1.21 to
 // 0.94 ms with this kernel and the range pass above (a thread per key before).
-__global__ void __launch_bounds__(kAsmTpb) k_conv_sum(const unsigned long long* __restrict__ keys,
-                                                     const int* __restrict__ perm, const int* __restrict__ start,
-                                                     int count, int col_bits, const double* __restrict__ vals,
+__global__ void __launch_bounds__(kAsmTpb) k_conv_sum(MergedKeys k, const double* __restrict__ vals,
                                                      int* rows_out, int* cols_out, double* vals_out)
 {
   const long long e = (long long)blockIdx.x * kAsmTpb + threadIdx.x;
   const int u = (int)(e / 9), q = (int)(e % 9);
-  if (u >= count) return;
-  const int s = start[u], end = start[u + 1];
-  if (q < 2) {
-    const unsigned long long k = keys[s];
-    if (q == 0)
-      rows_out[u] = (int)(k >> col_bits);
-    else
-      cols_out[u] = (int)(k & ((1ull << col_bits) - 1ull));
-  }
+  if (u >= k.count) return;
+  const int s = k.start[u], end = k.start[u + 1];
+  if (q == 0) rows_out[u] = k.rows[u];
+  if (q == 1) cols_out[u] = k.cols[u];
   double a = 0.0;
   for (int t = s; t < end; t += 4) {
     double v[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = t + k < end ? __ldcs(vals + 9 * (size_t)perm[t + k] + q) : 0.0;
+    for (int j = 0; j < 4; ++j) v[j] = t + j < end ? __ldcs(vals + 9 * (size_t)k.perm[t + j] + q) : 0.0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (t + k < end) a = a + v[k];
+    for (int j = 0; j < 4; ++j)
+      if (t + j < end) a = a + v[j];
   }
   vals_out[e] = a;
 }
@@ -172,6 +174,7 @@ MergedKeys merge_keys(maspcg_handle* h, const int* rows, const int* cols, int n)
     while (b < 32 && (v >> b) != 0u) ++b;
     return b;
   };
+  if (row_sort_triplets(h, rows, cols, n, fl[1], out)) return out;
   const int col_bits = bits((unsigned)fl[2]), key_bits = col_bits + bits((unsigned)fl[1]);
   k_conv_keys<<<grid, kAsmTpb, 0, st>>>(rows, cols, n, col_bits, k0, i0); MLAUNCHED(h);
   size_t need = 0;
@@ -190,13 +193,16 @@ MergedKeys merge_keys(maspcg_handle* h, const int* rows, const int* cols, int n)
   MCK(cudaStreamSynchronize(st));
   const int count = last[0] + last[1];
   h->asm_start.resize((size_t)count + 1);
-  k_conv_starts<<<grid, kAsmTpb, 0, st>>>(heads, pos, n, h->asm_start.get()); MLAUNCHED(h);
+  // (the keys' first copy is free by now: it takes the rows and columns)
+  int* urow = reinterpret_cast<int*>(k0);
+  int* ucol = urow + n;
+  k_conv_starts<<<grid, kAsmTpb, 0, st>>>(heads, pos, k1, n, col_bits, h->asm_start.get(), urow, ucol); MLAUNCHED(h);
   MCK(cudaGetLastError());
-  out.keys = k1;
+  out.rows = urow;
+  out.cols = ucol;
   out.perm = i1;
   out.start = h->asm_start.get();
   out.count = count;
-  out.col_bits = col_bits;
   return out;
 }
 
@@ -205,8 +211,8 @@ int convert_bcoo(maspcg_handle* h, const int* rows, const int* cols, const doubl
 {
   const MergedKeys k = merge_keys(h, rows, cols, n);
   if (k.count == 0) return 0;
-  k_conv_sum<<<ceil_div(9LL * k.count, kAsmTpb), kAsmTpb, 0, h->stream>>>(k.keys, k.perm, k.start, k.count, k.col_bits,
-                                                                          vals, rows_out, cols_out, vals_out);
+  k_conv_sum<<<ceil_div(9LL * k.count, kAsmTpb), kAsmTpb, 0, h->stream>>>(k, vals, rows_out, cols_out,
+                                                                          vals_out);
   MLAUNCHED(h);
   MCK(cudaGetLastError());
   return k.count;

@@ -108,8 +108,8 @@ __global__ void __launch_bounds__(kGalTpb) k_gal_sum(MergedKeys k, const unsigne
   const int u = (int)(e / 9), q = (int)(e % 9), t = q / 3 + 3 * (q % 3);
   if (u >= k.count) return;
   const int s = k.start[u], end = k.start[u + 1];
-  if (q == 0) rows_out[u] = (int)(k.keys[s] >> k.col_bits);
-  if (q == 1) cols_out[u] = (int)(k.keys[s] & ((1ull << k.col_bits) - 1ull));
+  if (q == 0) rows_out[u] = k.rows[u];
+  if (q == 1) cols_out[u] = k.cols[u];
   double a = 0.0;
   bool finite = true;
   for (int j = s; j < end; j += 4) {

@@ -226,10 +226,10 @@ struct maspcg_handle {
   maspcg::DBuf<int> int_of_row, row_of_int;
   maspcg::DBuf<int> rowptr, colidx;
   maspcg::DBuf<double> val64;     // row-major 3x3 blocks
-  maspcg::DBuf<float> val32;      // tiles of 32 blocks, element-major: (t/32)*288 + 32e + t%32
+  maspcg::DBuf<float> val32;      // tiles of 32 blocks, element-major: (t/32)*288 + 32e + t%32 (FP32, mixed)
   maspcg::DBuf<unsigned short> val_lo;  // MASPCG_MATRIX_F32_SPLIT: BF16 of A - A32, laid out as val32
   maspcg::DBuf<unsigned long long> keys, keys_sorted;
-  maspcg::DBuf<int> kv, kv_sorted, seg_head, seg_start, row_count;
+  maspcg::DBuf<int> kv, kv_sorted, seg_head, seg_start, row_count, row_start;
   maspcg::DBuf<double> in_vals;
   maspcg::DBuf<int> in_rows, in_cols;
 
@@ -339,15 +339,24 @@ void bcoo_gradient(maspcg_handle* h, const int* rows, const int* cols, int n, co
 void modulus_gradient(maspcg_handle* h, const int* rows, const int* cols, const double* vals, int ntet, int bpt,
                       const double* lam, const double* x, const double* E, double* gE);
 
+// rowsort.cu: the merge order by row buckets; false leaves it to a radix sort.
+// row_sort_matrix fills rowptr, colidx, seg_start, kv_sorted, m_valid and nnzb
+// of the symmetric structure; row_sort_triplets the order of n triplets with
+// rows up to last_row.
+struct MergedKeys;
+bool row_sort_matrix(maspcg_handle* h, const int* rows, const int* cols, int n);
+bool row_sort_triplets(maspcg_handle* h, const int* rows, const int* cols, int n, int last_row, MergedKeys& out);
+
 // assemble.cu (device pointers; returns the unique count / the type counts)
-// The triplets' order and runs by key (row << col_bits) + col: entries
-// perm[start[u]] .. perm[start[u + 1] - 1], in input order, belong to unique key
-// u, whose key is keys[start[u]] (handle scratch).
+// The triplets' order and runs by (row, col): entries perm[start[u]] ..
+// perm[start[u + 1] - 1], in input order, belong to unique block u of row
+// rows[u] and column cols[u] (handle scratch).
 struct MergedKeys {
-  const unsigned long long* keys;
+  const int* rows;
+  const int* cols;
   const int* perm;
   const int* start;
-  int count, col_bits;
+  int count;
 };
 MergedKeys merge_keys(maspcg_handle* h, const int* rows, const int* cols, int n);
 int convert_bcoo(maspcg_handle* h, const int* rows, const int* cols, const double* vals, int n, int* rows_out,

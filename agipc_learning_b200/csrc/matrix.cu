@@ -91,7 +91,8 @@ __global__ void k_fill_structure(const unsigned long long* __restrict__ keys, co
 // One CTA per tile of 32 stored blocks, a thread per element: the input blocks
 // of the element summed in sorted (= input) order, fetched four ahead.  Nine
 // consecutive threads read a block's 72 bytes and write its FP64 values; the
-// FP32 tile is transposed in shared memory and written in one run.
+// FP32 tile (null in the reference precision, which does not read it) is
+// transposed in shared memory and written in one run.
 // Bound by the scattered input blocks.  With the row maps formed on the device the
 // matrix of the 64^3 contact system is built in 0.87 ms, 1.31 with a thread per
 // block and the maps copied from the host.
@@ -125,6 +126,7 @@ __global__ void __launch_bounds__(kFillTpb) k_fill_values(const int* __restrict_
     }
     val64[9 * (size_t)u + q] = a;
   }
+  if (!val32) return;  // uniform
   const float hi = (float)a;
   hi_s[32 * q + b] = hi;  // tiles of 32 blocks, element-major
   // the remainder a - hi is exact in FP64; its BF16 rounding carries A to
@@ -277,11 +279,15 @@ __global__ void __launch_bounds__(32 * kAbdWarps) k_abd_inverse(const int* __res
       inv64[144 * (size_t)bdy + 12 * r + lane - 12] = ok ? a[r] : (r == lane - 12 ? 1.0 : 0.0);
 }
 
+// The reference precision runs on the FP64 values alone.
+bool runs_fp32(const maspcg_handle* h) { return h->cfg.precision != MASPCG_PREC_REFERENCE; }
+
 // The merged values of the current structure from the input blocks.
 void fill_values(maspcg_handle* h, const double* vals)
 {
   k_fill_values<<<ceil_div(h->nnzb, 32), kFillTpb, 0, h->stream>>>(
-      h->kv_sorted.get(), h->seg_start.get(), h->nnzb, h->m_valid, vals, h->val64.get(), h->val32.get(),
+      h->kv_sorted.get(), h->seg_start.get(), h->nnzb, h->m_valid, vals, h->val64.get(),
+      runs_fp32(h) ? h->val32.get() : nullptr,
       h->cfg.matrix_form == MASPCG_MATRIX_F32_SPLIT ? h->val_lo.get() : nullptr);
   MLAUNCHED(h);
   MCK(cudaGetLastError());
@@ -295,39 +301,16 @@ size_t cub_bytes_sort(int m, int end_bit)
   return b;
 }
 
-}  // namespace
-
-void build_internal_matrix(maspcg_handle* h, const double* vals, const int* rows, const int* cols, int n)
+// The structure by a stable radix sort of (row, col) keys (rows of any length).
+void radix_sort_matrix(maspcg_handle* h, const int* rows, const int* cols, int n)
 {
   cudaStream_t st = h->stream;
-  const int nb = h->nb;
-  // ---- internal row order
-  h->mas_layout = (h->cfg.preconditioner == MASPCG_PRECOND_MAS32 || h->cfg.preconditioner == MASPCG_PRECOND_MAS16) &&
-                  h->has_graph && h->nv > 0;
-  int nb_int = nb;
-  if (h->mas_layout) {
-    MREQ(h->fem_off + h->nv <= nb, MASPCG_ERR_INVALID_ARGUMENT, "FEM range exceeds the block rows");
-    nb_int = nb + h->c0 - h->nv;
-  }
-  h->nb_int = nb_int;
-  h->int_of_row.resize(nb);
-  h->row_of_int.resize(nb_int);
-  k_row_maps<<<ceil_div(std::max(nb, nb_int), kTpb), kTpb, 0, st>>>(
-      nb, nb_int, h->mas_layout ? h->fem_off : nb, h->mas_layout ? h->nv : 0, h->mas_layout ? h->c0 : 0, h->rmp.get(),
-      h->pmr.get(), h->int_of_row.get(), h->row_of_int.get()); MLAUNCHED(h);
-
-  // ---- keys
+  const int nb = h->nb, nb_int = h->nb_int, m = 2 * n;
   int bits = 1;
   while ((1ll << bits) <= nb_int) ++bits;
   MREQ(2 * bits <= 62, MASPCG_ERR_CAPACITY, "too many block rows");
-  const int m = 2 * n;
-  h->keys.resize(m);
   h->keys_sorted.resize(m);
-  h->kv.resize(m);
-  h->kv_sorted.resize(m);
   h->seg_head.resize(m);
-  h->seg_start.resize(m + 1);
-  h->failed.resize(8);
   MCK(cudaMemsetAsync(h->failed.get(), 0, sizeof(int) * 8, st));
   k_make_keys<<<ceil_div(n, kTpb), kTpb, 0, st>>>(rows, cols, n, nb, h->int_of_row.get(), bits, h->keys.get(),
                                                  h->kv.get(), h->failed.get()); MLAUNCHED(h);
@@ -356,17 +339,52 @@ void build_internal_matrix(maspcg_handle* h, const double* vals, const int* rows
   h->m_valid = m_valid;
   h->nnzb = nnzb;
   h->colidx.resize(nnzb, 4);  // 16-byte tail for TMA bulk copies
-  h->val64.resize((size_t)9 * nnzb, 2);
-  h->val32.resize((size_t)9 * (((size_t)nnzb + 31) / 32 * 32));
-  if (h->cfg.matrix_form == MASPCG_MATRIX_F32_SPLIT) h->val_lo.resize(h->val32.n);
-  h->row_count.resize(nb_int + 1);
-  h->rowptr.resize(nb_int + 1);
   MCK(cudaMemsetAsync(h->row_count.get(), 0, sizeof(int) * (nb_int + 1), st));
   k_fill_structure<<<ceil_div(m, kTpb), kTpb, 0, st>>>(h->keys_sorted.get(), h->seg_head.get(), h->kv.get(), m, bits,
                                                       h->colidx.get(), h->seg_start.get(), h->row_count.get()); MLAUNCHED(h);
   // rowptr = exclusive scan of the per-row counts (the extra entry gives nnzb)
   tb = h->cub_tmp.cap;
   MCK(cub::DeviceScan::ExclusiveSum(h->cub_tmp.get(), tb, h->row_count.get(), h->rowptr.get(), nb_int + 1, st));
+  MCK(cudaGetLastError());
+}
+
+}  // namespace
+
+void build_internal_matrix(maspcg_handle* h, const double* vals, const int* rows, const int* cols, int n)
+{
+  cudaStream_t st = h->stream;
+  const int nb = h->nb;
+  // ---- internal row order
+  h->mas_layout = (h->cfg.preconditioner == MASPCG_PRECOND_MAS32 || h->cfg.preconditioner == MASPCG_PRECOND_MAS16) &&
+                  h->has_graph && h->nv > 0;
+  int nb_int = nb;
+  if (h->mas_layout) {
+    MREQ(h->fem_off + h->nv <= nb, MASPCG_ERR_INVALID_ARGUMENT, "FEM range exceeds the block rows");
+    nb_int = nb + h->c0 - h->nv;
+  }
+  h->nb_int = nb_int;
+  h->int_of_row.resize(nb);
+  h->row_of_int.resize(nb_int);
+  k_row_maps<<<ceil_div(std::max(nb, nb_int), kTpb), kTpb, 0, st>>>(
+      nb, nb_int, h->mas_layout ? h->fem_off : nb, h->mas_layout ? h->nv : 0, h->mas_layout ? h->c0 : 0, h->rmp.get(),
+      h->pmr.get(), h->int_of_row.get(), h->row_of_int.get()); MLAUNCHED(h);
+
+  // ---- structure: row buckets, or a radix sort where a row is too long
+  const int m = 2 * n;
+  h->keys.resize(m);
+  h->kv.resize(m);
+  h->kv_sorted.resize(m);
+  h->seg_start.resize(m + 1);
+  h->failed.resize(8);
+  MCK(cudaMemsetAsync(h->failed.get(), 0, sizeof(int) * 8, st));
+  h->row_count.resize(nb_int + 1);
+  h->rowptr.resize(nb_int + 1);
+  if (!row_sort_matrix(h, rows, cols, n)) radix_sort_matrix(h, rows, cols, n);
+  const int nnzb = h->nnzb;
+  h->val64.resize((size_t)9 * nnzb, 2);
+  const size_t tiled = (size_t)9 * (((size_t)nnzb + 31) / 32 * 32);
+  if (runs_fp32(h)) h->val32.resize(tiled);
+  if (h->cfg.matrix_form == MASPCG_MATRIX_F32_SPLIT) h->val_lo.resize(tiled);
   if (h->vals_pending) {  // host values copied on the side stream
     MCK(cudaStreamWaitEvent(st, h->ev_join, 0));
     h->vals_pending = false;
