@@ -1437,8 +1437,30 @@ double time_stage(maspcg_handle* h, int stage, int repeats)
   }
 }
 
+// Whether a solve's iterations run as programmatic dependent launches without
+// MASPCG_FLAG_PDL.  In the reference precision the kernels of an iteration are
+// one chain, and the next one's launch and prologue hide behind the last one's
+// tail: 29.5 -> 27.5 us per iteration at 8,000 rows, 47.1 -> 44.0 on the hybrid
+// system (22,000), 75.0 -> 74.4 at 101,565.  Without MAS the chain is the SpMV and
+// two vector updates, and on large systems the waiting CTAs cost more than that
+// (23.5 -> 22.0 us at 21,952 rows, 34.6 -> 37.5 at 64,000).  The overlapped
+// schedule of the other precisions loses by it below 100,000 rows (44.9 -> 48.2 at
+// 64,000) and gains nothing beyond.
+bool pdl_pays(const maspcg_handle* h)
+{
+  return h->cfg.precision == MASPCG_PREC_REFERENCE && (h->mas_layout || h->nb_int <= 32768);
+}
+
+struct PdlScope {
+  maspcg_handle* h;
+  bool was;
+  explicit PdlScope(maspcg_handle* h_) : h(h_), was(h_->use_pdl) { h->use_pdl = was || pdl_pays(h); }
+  ~PdlScope() { h->use_pdl = was; }
+};
+
 void solve(maspcg_handle* h, const double* b_int, double* x_int, maspcg_result* res)
 {
+  const PdlScope pdl(h);
   switch (h->cfg.precision) {
     case MASPCG_PREC_REFERENCE: {
       Engine<double, double, double> e(h);
