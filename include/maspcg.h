@@ -131,7 +131,8 @@ typedef enum {
 /* Kernel-schedule choices (bits of maspcg_config.flags); results do not depend
  * on them beyond floating-point summation order. */
 typedef enum {
-  MASPCG_FLAG_PDL = 1,                 /* launch iteration kernels with programmatic dependent launch */
+  MASPCG_FLAG_PDL = 1,                 /* launch iteration kernels with programmatic dependent launch (without it:
+                                          in MASPCG_PREC_REFERENCE only, where it pays) */
   MASPCG_FLAG_APPLY_STAGED2 = 2,       /* 16-bit level-0 apply: two TMA slots per warp */
   MASPCG_FLAG_APPLY_DIRECT = 4,        /* 16-bit level-0 apply: records staged by per-lane loads, no TMA */
   MASPCG_FLAG_SEQUENTIAL_COARSE = 8,   /* run the MAS coarse levels before the level-0 apply, not beside it
