@@ -210,3 +210,29 @@ def test_body_inverses_and_apply(bodies, precision):
         tol = 144 * np.finfo(np.float64).eps * np.linalg.cond(A) + 4 * eps * np.linalg.cond(A)
         assert np.linalg.norm(z[12 * k:12 * k + 12] - zk) <= tol * np.linalg.norm(zk), k
     assert np.allclose(z[12 * bodies:], b[12 * bodies:] / 2, rtol=1e-6)
+
+
+@pytest.mark.parametrize("long_row", [31, 33, 255, 257, 1023, 1024, 1025, 2600])
+def test_rows_around_the_bucket_limits(long_row):
+    """One row of the given number of triplets (a bucket's sort widths, and the
+    limit beyond which a radix sort takes over) among short ones, every third
+    triplet repeated: the merge bit-exact, the matrix product to the FP64 bound."""
+    rng = np.random.default_rng(long_row)
+    nb = 3000
+    distinct = nb - 1 - rng.permutation(nb - 8)[:max(long_row * 2 // 3, 1)]
+    hub = np.concatenate([distinct, distinct[:long_row - len(distinct)]])
+    r = np.concatenate([np.full(long_row, 7), np.arange(nb), rng.integers(0, 7, 500)])
+    c = np.concatenate([hub, np.arange(nb), rng.integers(7, nb, 500)])
+    order = rng.permutation(len(r))
+    r, c = r[order].astype(np.int32), c[order].astype(np.int32)
+    v = rng.standard_normal((len(r), 9))
+    x = rng.standard_normal(3 * nb)
+    ro, co, vo = oracle.convert_triplets(r, c, v)
+    with MasPcg(preconditioner="none", precision="reference") as m:
+        rg, cg, vg = m.convert_bcoo(r, c, v)
+        m.set_matrix(v, r, c, nb)
+        y = m.spmv(x)
+    assert np.array_equal(rg, ro) and np.array_equal(cg, co) and np.array_equal(vg, vo)
+    ref = oracle.sym_spmv(1.0, v, r, c, x)
+    mag = oracle.sym_spmv(1.0, np.abs(v), r, c, np.abs(x))
+    assert np.all(np.abs(y - ref) <= 3 * 3000 * np.finfo(np.float64).eps * mag + 1e-300)
