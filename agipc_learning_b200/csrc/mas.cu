@@ -347,13 +347,14 @@ __device__ __forceinline__ void b_frag(const unsigned short* part, int K, int g,
   }
 }
 
-// Sum of the three split-term columns of 6 accumulator tiles into out[96]:
+// Sum of the three split-term columns of accumulator tiles into out (16 rows each):
 // thread (g, q = 0) holds columns 0-1 of rows g and g + 8, thread (g, 1)
 // column 2.
-__device__ __forceinline__ void reduce_columns(float acc[6][4], float* out, int g, int q)
+template <int kTilesUp>
+__device__ __forceinline__ void reduce_columns(float acc[kTilesUp][4], float* out, int g, int q)
 {
 #pragma unroll
-  for (int I = 0; I < 6; ++I) {
+  for (int I = 0; I < kTilesUp; ++I) {
     float t0 = acc[I][0] + acc[I][1], t1 = acc[I][2] + acc[I][3];
     t0 += __shfl_down_sync(kFull, t0, 1);
     t1 += __shfl_down_sync(kFull, t1, 1);
@@ -406,7 +407,7 @@ __device__ __forceinline__ void domain_apply16(const TI* rec, unsigned char* scr
         M::mma(acc[I], a, b0, b1);
       }
     }
-    reduce_columns(acc, vf, g, q);
+    reduce_columns<6>(acc, vf, g, q);
   }
   __syncwarp();
   v[0] = vf[3 * lane];
@@ -437,7 +438,7 @@ __device__ __forceinline__ void domain_apply16(const TI* rec, unsigned char* scr
         M::mma(acc[J], a, b0, b1);
       }
     }
-    reduce_columns(acc, vf, g, q);
+    reduce_columns<6>(acc, vf, g, q);
   }
   __syncwarp();
   const float back = fi1 * fi2;
@@ -545,14 +546,14 @@ __global__ void k_coarse_spans(CoarseLevels a)
   }
 }
 
-// Threads of a coarse domain's CTA: a warp per 16x16 tile of a 16-bit record
-// (one 16-byte load per thread holds it), a thread per block of the wrapped
-// diagonals of an FP32 one.
+// Threads of a coarse domain's CTA: one 16-byte load per thread fetches a 16-bit
+// record (21 tiles of 16x16, six warps apply them), a thread per block of the
+// wrapped diagonals of an FP32 one.
 template <typename TI, int kB>
 constexpr int coarse_threads() { return sizeof(TI) == 2 ? 32 * kTiles16 : kDiags * kB; }
 
 // One coarse domain per CTA: R of its nodes, then Z = M R with the whole record
-// in registers, loaded before R is needed.  Latency is all that counts here
+// on the chip, loaded before R is needed.  Latency is all that counts here
 // (a few hundred domains of 10-20 KB): a few dependent loads and barriers,
 // where the form before walked up the hierarchy through counters that the CTAs
 // waited on, and one warp applied a domain: 15 us for the 266 coarse domains of
@@ -573,9 +574,10 @@ __global__ void __launch_bounds__(coarse_threads<TI, kB>(), 2) k_coarse_levels(C
   // up (the partial products afterwards)
   extern __shared__ __align__(16) float coarse_smem[];
   float* stage = coarse_smem + 2 * 3 * kCoarseOnChip;
-  __shared__ float xs[kN], vs[kN];
+  __shared__ float xs[kN], vs[kN], norm[2];
+  __shared__ __align__(4) unsigned short part[kTiled ? 3 * kPartStride : 1];
   float* p1 = stage;
-  float* p2 = stage + (kTiled ? kTiles16 * 16 : kD * kN);
+  float* p2 = stage + kD * kN;
   static_assert(2 * kDiags * 3 * kBank <= kCoarseStage, "partial products share the stage");
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
   const int g = a.lv.domains - 1 - blockIdx.x;  // the top levels, with most below them, start first
@@ -674,57 +676,59 @@ __global__ void __launch_bounds__(coarse_threads<TI, kB>(), 2) k_coarse_levels(C
     }
     if (tid >= 3 * min(kB, a.lv.count[l] - (kB * g - a.lv.begin[l])) && tid < kN) xs[tid] = 0.f;
   }
-  if (kTiled && tid < kN) vs[tid] = xs[tid] * sc;
+  if constexpr (kTiled) {
+    if (tid < kN) vs[tid] = xs[tid] * sc;  // (by the thread that wrote xs[tid], or after its barrier)
+    reinterpret_cast<uint4*>(stage)[tid] = rec;
+  }
   __syncthreads();
   // ---- Z = M R
   float y = 0.f;
   if constexpr (kTiled) {
-    // M = S V^T V S, warp w holding tile (I, J) of V: lane 2r + h its row r,
-    // columns 8 half .. 8 half + 7 (inv16_pos swaps the halves of rows 4-7 and
-    // 12-15).  FP32 products and sums of the exactly widened elements.
-    int I = 0;
-    while ((I + 1) * (I + 2) / 2 <= w) ++I;
-    const int J = w - I * (I + 1) / 2, row = lane >> 1, half = (lane ^ (lane >> 3)) & 1;
-    const uint32_t u[4] = {rec.x, rec.y, rec.z, rec.w};
-    float V[8];
+    // The products of domain_apply16 in its order, so a domain's Z is the same
+    // to the bit whichever kernel forms it: warp I < 6 holds row tile I of pass
+    // 1 and column tile I of pass 2, and warp 0 splits the vector for both.
+    // (Plain FP32 products, a warp per tile, were 1% faster on whole solves,
+    // 75.2 against 76.0 ms at 64,000 rows.  Where FP32 values barely converge,
+    // as with dense contacts on small boxes, that rounding decided between
+    // 4,034 iterations and the cap.)
+    using M = Mma16<TI>;
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(stage);
+    const int g8 = lane >> 2, q4 = lane & 3, m8 = lane >> 3, rr = lane & 7;
+    const uint32_t off_n = ((((m8 & 1) << 3) + rr) << 5) + ((((m8 >> 1) ^ (rr >> 2)) & 1) << 4);
+    const uint32_t off_t = ((((m8 >> 1) << 3) + rr) << 5) + ((((m8 & 1) ^ (rr >> 2)) & 1) << 4);
+    float back = 1.f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) V[k] = Mma16<TI>::from16((unsigned short)(u[k / 2] >> (16 * (k & 1))));
-    float t = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) t = fmaf(V[k], vs[16 * J + 8 * half + k], t);
-    t += __shfl_xor_sync(kFull, t, 1);
-    if ((lane & 1) == 0) p1[16 * w + row] = t;
-    __syncthreads();
-    if (tid < kN) {
-      const int R = tid >> 4;
-      float v = 0.f;
-      for (int q = 0; q <= R; ++q) v += p1[16 * (R * (R + 1) / 2 + q) + (tid & 15)];
-      vs[tid] = v;  // every warp has read its S R
-    }
-    __syncthreads();
-    t = vs[16 * I + row];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) V[k] *= t;
-    // column sums over the tile's 16 rows: halving exchanges over row bits 0,
-    // 1 and 3, then row bit 2, whose partner lane with the same half is lane ^ 9
-#pragma unroll
-    for (int n = 4; n >= 1; n >>= 1) {
-      const int mask = n == 4 ? 2 : (n == 2 ? 4 : 16);
-      const bool up = (lane & mask) != 0;
-#pragma unroll
-      for (int k = 0; k < n; ++k) {
-        const float keep = up ? V[k + n] : V[k], give = up ? V[k] : V[k + n];
-        V[k] = keep + __shfl_xor_sync(kFull, give, mask);
+    for (int pass = 0; pass < 2; ++pass) {
+      if (w == 0) {
+        float v[3] = {vs[3 * lane], vs[3 * lane + 1], vs[3 * lane + 2]};
+        if constexpr (M::kNormalize) {
+          float f, fi;
+          pow2_normalizer(v, f, fi);
+          v[0] *= f;
+          v[1] *= f;
+          v[2] *= f;
+          if (lane == 0) norm[pass] = fi;
+        }
+        split_store<TI>(part, lane, v);
       }
+      __syncthreads();
+      if (w < kN / 16) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int K = pass == 0 ? 0 : w; K < (pass == 0 ? w + 1 : kN / 16); ++K) {
+          uint32_t b0, b1, t[4];
+          b_frag(part, K, g8, q4, b0, b1);
+          if (pass == 0)
+            ldsm(base + (uint32_t)((w * (w + 1) / 2 + K) * 512) + off_n, t);
+          else
+            ldsm_t(base + (uint32_t)((K * (K + 1) / 2 + w) * 512) + off_t, t);
+          M::mma(acc, t, b0, b1);
+        }
+        reduce_columns<1>(&acc, vs + 16 * w, g8, q4);
+      }
+      __syncthreads();
     }
-    V[0] += __shfl_xor_sync(kFull, V[0], 9);
-    if ((lane & 8) == 0) p2[16 * w + 8 * half + ((lane & 2) << 1) + ((lane & 4) >> 1) + (lane >> 4)] = V[0];
-    __syncthreads();
-    if (tid < kN) {
-      const int C = tid >> 4;
-      for (int q = C; q < 6; ++q) y += p2[16 * (q * (q + 1) / 2 + C) + (tid & 15)];
-      y *= sc;
-    }
+    if constexpr (M::kNormalize) back = norm[0] * norm[1];
+    if (tid < kN) y = vs[tid] * back * sc;
   } else {
     // the symmetric inverse: block (ln, ln + d) serves both triangles; the
     // products and the order of the sums are those of domain_apply

@@ -153,6 +153,41 @@ def test_apply_on_fragmented_hierarchies(n, precision, inverse):
     assert np.linalg.norm(z - zo) <= 1e-5 * np.linalg.norm(zo)
 
 
+@pytest.mark.parametrize("inverse", ["bf16", "fp16", "fp32"])
+def test_coarse_domains_apply_as_level_0(inverse):
+    """Without neighbours every vertex is a node of its own on every level, so
+    the coarse domains repeat level 0's two, and z is three equal terms; with
+    each bank one component and residuals that cancel in it, z is level 0's
+    alone.  The two differ by exactly that factor when the coarse levels form a
+    domain's product as level 0 does, rounding included."""
+    rng = np.random.default_rng(5)
+    nb = 64
+    rows, cols, vals = [], [], []
+    for bank in (0, 32):
+        A = rng.standard_normal((96, 96))
+        A = A @ A.T / 96 + np.diag(10.0 ** rng.uniform(-2, 2, 96))
+        for i in range(32):
+            for j in range(i, 32):
+                rows.append(bank + i), cols.append(bank + j), vals.append(A[3 * i:3 * i + 3, 3 * j:3 * j + 3].T.reshape(9))
+    r = rng.integers(-1000, 1000, (2, 32, 3)).astype(np.float64)
+    r[:, 31] -= r.sum(axis=1)
+    ident = np.arange(nb, dtype=np.int32)
+    chain = [[u for u in (v - 1, v + 1) if 0 <= u < nb and u // 32 == v // 32] for v in range(nb)]
+    z = []
+    for lists in ([[]] * nb, chain):
+        num = np.array([len(q) for q in lists], np.uint32)
+        start = (np.cumsum(num) - num).astype(np.uint32)
+        with MasPcg(precision="mixed", inverse=inverse) as m:
+            m.set_graph(nb, 0, start, num, np.array([u for q in lists for u in q], np.uint32), ident, ident)
+            m.set_contacts(np.zeros((0, 4), np.int32))
+            m.set_matrix(np.array(vals), np.array(rows, np.int32), np.array(cols, np.int32), nb)
+            m.build()
+            assert m.info()["levelnum"] == 3
+            z.append(m.apply_preconditioner(r.reshape(-1)).astype(np.float32))
+    assert np.any(z[1] != 0)
+    assert np.array_equal(z[0], z[1] + (z[1] + z[1]))
+
+
 @pytest.mark.parametrize("n", [1, 33, 2049])
 def test_block_gradient_checks_every_index(n):
     """An index outside the system in the last block is refused before anything
