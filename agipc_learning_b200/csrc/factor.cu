@@ -1,34 +1,178 @@
-// factor.cu -- the MAS domain inverses: gather, FP64 Cholesky and store of one
-// domain per CTA (MAS32: 96x96; CEMAS16: 48x48).
+// factor.cu -- the MAS domain inverses: gather, FP64 factorisation and store of
+// one domain per CTA (MAS32: 96x96; CEMAS16: 48x48).
 //
 // The reference inverts each domain by Gauss-Jordan elimination without
 // pivoting (__inverse6_P96x96, TraditionalMAS32Preconditioner.cu:1099-1146).
-// The same inverse comes here from A = L L^T and W = L^-1: FP32 storage takes
-// W^T W, 16-bit storage the scaled factor W S^-1 itself.  A pivot <= 0 or not
-// finite counts the domain as failed and stands as 1, as in the elimination
-// (both eliminate the same pivots in the same order).
-//
-// The lower triangle lives in shared memory as 8x8 FP64 tiles (40 KB for a
-// 96x96 domain), and everything but the 8x8 diagonal tiles runs on the FP64
-// tensor instruction mma.m8n8k4.  Each step k: the tiles below the diagonal
-// times L_kk^-T, then the trailing tiles less L_ik L_jk^T, while the first warp
-// updates the next diagonal tile first and factors it (its chain of eight
-// pivots is the longest of the step).  W needs no second factorisation-like
-// sweep: with H_kj = -L_kj L_jj^-1, row i of W is
-//   W_ii = L_ii^-1,  W_ij = sum over k = j+1 .. i of W_ik H_kj,
-// so each warp runs whole rows in registers and the rows need three barriers.
-// Bound by the chain of twelve steps (the FP64 pipe is 34% busy with five CTAs per
-// SM): 0.73 ms for 8,192 domains in BF16 storage and 0.38 for 3,174 in FP32, where
-// a gather and a 3x3-block Cholesky took 2.7 and Gauss-Jordan steps 1.5.
-#include <type_traits>
-
+// FP32 storage runs that elimination (k_domain_eliminate).  16-bit storage
+// takes the same pivots through A = L L^T and keeps the scaled factor W S^-1,
+// W = L^-1 (k_domain_invert).  A pivot <= 0 or not finite counts the domain as
+// failed and stands as 1 in both.
 #include "maspcg_internal.cuh"
 
 namespace maspcg {
 namespace {
 
+// ---- FP32 storage ----------------------------------------------------------
+
+constexpr int kElimSide = 6;  // a thread's square of the matrix: two by two blocks
+
+// In-place Gauss-Jordan of the whole matrix in registers, kB/2 x kB/2 threads
+// with a 6x6 square each.  A step publishes the pivot's row and column, waits
+// once, and is 36 multiply-adds per thread with two CTAs per SM to hide each
+// other's wait.  Every element takes the reference's operations in the
+// reference's order: x - (m / pivot) p per step, so the result is that of the
+// elimination on the matrix as it is -- also where CEMAS16's assembly rules
+// leave a coarse diagonal block unsymmetric, which a Cholesky factor of one
+// triangle does not see (6e-3 of an inverse's largest entry on such a domain).
+// Bound by the chain of steps (wait, reciprocal, 36 multiply-adds, next pivot).
+// Whole factor stage with coarse sums: 1.07 ms for 3,347 domains of 96 rows and
+// 0.68 for 7,675 of 48, where a 3x3 block per thread (1,024 and 512 threads, one
+// CTA per SM) took 1.74 and 1.14, and the tensor-tile Cholesky below with a
+// closing W^T W 0.89 and 0.68.
 template <int kB>
-constexpr int factor_threads() { return kB == 32 ? 128 : 64; }
+__global__ void __launch_bounds__(kB * kB / 4, kB == 32 ? 2 : 8) k_domain_eliminate(FactorArgs a, int dom_offset)
+{
+  constexpr int kG = kB / 2, kT = kG * kG, kN = 3 * kB, kS = kElimSide;
+  constexpr int kDiag = kB / 2 + 1, kElems = kDiag * 9 * kB;
+  __shared__ __align__(16) double half[kN / 2 * kN];  // half the rows at a time; the record afterwards
+  __shared__ __align__(16) double row[2][kN], col[2][kN];
+  __shared__ double recip[2];
+  __shared__ int rp[kB + 1], fail;
+  static_assert(kElems * sizeof(float) <= sizeof(half) && kElems % 4 == 0, "the record fits the half matrix");
+  const int tid = threadIdx.x, ty = tid / kG, tx = tid % kG;
+  const int dom = blockIdx.x + dom_offset, d0 = a.lv.dom_begin[1];
+  if (tid == 0) fail = 0;
+
+  // ---- the domain's blocks (rows 6 ty, columns 6 tx)
+  double acc[kS][kS];
+  if (dom < d0) {
+    const int row0 = a.fem_off + kB * dom;  // first internal row
+    for (int e = tid; e <= kB; e += kT) rp[e] = a.rowptr[row0 + e];
+    for (int h = 0; h < 2; ++h) {
+      for (int e = tid; e < kN / 2 * kN / 2; e += kT) reinterpret_cast<double2*>(half)[e] = make_double2(0.0, 0.0);
+      __syncthreads();
+      const int r0 = h * kG, end = rp[r0 + kG];
+      for (int t = rp[r0] + tid; t < end; t += kT) {  // a thread per block (a merged block appears once)
+        const int bc = a.colidx[t] - row0;
+        if (bc < 0 || bc >= kB) continue;
+        int lo = r0, hi = r0 + kG;  // row lo: rp[lo] <= t < rp[lo + 1]
+        while (hi - lo > 1) {
+          const int mid = (lo + hi) >> 1;
+          if (rp[mid] <= t) lo = mid; else hi = mid;
+        }
+        if (kB == 16 && bc != lo) {
+          // CEMAS16 drops a pair whose slot order runs against its vertex order
+          const int* pm = a.pmr + kB * dom;
+          if ((pm[lo] < pm[bc]) != (lo < bc)) continue;
+        }
+        double* m = half + 3 * (lo - r0) * kN + 3 * bc;
+#pragma unroll
+        for (int e = 0; e < 9; ++e) m[e / 3 * kN + e % 3] = __ldcs(a.val64 + 9 * (size_t)t + e);
+      }
+      __syncthreads();
+      if (ty / (kG / 2) == h) {
+#pragma unroll
+        for (int i = 0; i < kS; ++i)
+#pragma unroll
+          for (int k = 0; k < kS; ++k) acc[i][k] = half[(kS * ty + i - h * kN / 2) * kN + kS * tx + k];
+      }
+      __syncthreads();
+    }
+  } else {
+#pragma unroll
+    for (int bi = 0; bi < 2; ++bi)
+#pragma unroll
+      for (int bk = 0; bk < 2; ++bk) {
+        const double* src = a.coarse64 + (((size_t)(dom - d0) * kB + 2 * ty + bi) * kB + 2 * tx + bk) * 9;
+#pragma unroll
+        for (int e = 0; e < 9; ++e) acc[3 * bi + e / 3][3 * bk + e % 3] = src[e];
+      }
+  }
+  if (ty == tx)  // padding slots: zero diagonal -> 1
+#pragma unroll
+    for (int i = 0; i < kS; ++i)
+      if (acc[i][i] == 0.0) acc[i][i] = 1.0;
+
+  // ---- elimination; two copies of the row and column, so one barrier a step
+  for (int q = 0; q < kG; ++q) {
+#pragma unroll
+    for (int c = 0; c < kS; ++c) {
+      const int b = c & 1;
+      if (tx == q) {
+#pragma unroll
+        for (int i = 0; i < kS; ++i) col[b][kS * ty + i] = acc[i][c];
+      }
+      if (ty == q) {
+#pragma unroll
+        for (int k = 0; k < kS; ++k) row[b][kS * tx + k] = acc[c][k];
+        if (tx == q) {
+          double pivot = acc[c][c];
+          if (!(pivot > 0.0) || !isfinite(pivot)) fail = 1, pivot = 1.0;
+          recip[b] = 1.0 / pivot;
+        }
+      }
+      __syncthreads();
+      const double inv = recip[b];
+      double f[kS];
+#pragma unroll
+      for (int i = 0; i < kS; ++i) f[i] = col[b][kS * ty + i] * inv;
+#pragma unroll
+      for (int k = 0; k < kS; ++k) {
+        const double p = row[b][kS * tx + k];
+#pragma unroll
+        for (int i = 0; i < kS; ++i) acc[i][k] = fma(-f[i], p, acc[i][k]);
+        if (ty == q) acc[c][k] = p * inv;
+      }
+      if (tx == q) {
+#pragma unroll
+        for (int i = 0; i < kS; ++i) acc[i][c] = -f[i];
+        if (ty == q) acc[c][c] = inv;
+      }
+    }
+  }
+  __syncthreads();
+  if (tid == 0 && fail) atomicAdd(a.failed, 1);
+
+  // ---- wrapped diagonals: block (l, (l + d) % kB) at [d][3i + j][l], the last
+  // diagonal for l < kB / 2 only
+  float* out = reinterpret_cast<float*>(half);
+#pragma unroll
+  for (int bi = 0; bi < 2; ++bi)
+#pragma unroll
+    for (int bk = 0; bk < 2; ++bk) {
+      const int l = 2 * ty + bi, d = (2 * tx + bk - l) & (kB - 1);
+      if (d > kB / 2) continue;
+      const bool zero = d == kB / 2 && l >= kB / 2;
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          // CEMAS16 stores the diagonal blocks with their lower elements
+          // taken from the upper ones (MASPreconditioner.cu:705-711)
+          const bool upper = kB == 16 && d == 0 && i > j;
+          const double v = upper ? acc[3 * bi + j][3 * bk + i] : acc[3 * bi + i][3 * bk + j];
+          out[(9 * d + 3 * i + j) * kB + l] = zero ? 0.f : (float)v;
+        }
+    }
+  __syncthreads();
+  float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.inv) + (size_t)dom * kElems);
+  for (int e = tid; e < kElems / 4; e += kT) dst[e] = reinterpret_cast<const float4*>(out)[e];
+}
+
+// ---- 16-bit storage --------------------------------------------------------
+//
+// The lower triangle lives in shared memory as 8x8 FP64 tiles (40 KB), and
+// everything but the 8x8 diagonal tiles runs on the FP64 tensor instruction
+// mma.m8n8k4.  Each step k: the tiles below the diagonal times L_kk^-T, then the
+// trailing tiles less L_ik L_jk^T, while the first warp updates the next
+// diagonal tile first and factors it (its chain of eight pivots is the longest
+// of the step).  W needs no second factorisation-like sweep: with
+// H_kj = -L_kj L_jj^-1, row i of W is
+//   W_ii = L_ii^-1,  W_ij = sum over k = j+1 .. i of W_ik H_kj,
+// so each warp runs whole rows in registers and the rows need three barriers.
+// Bound by the chain of twelve steps: 0.73 ms for 8,192 domains in BF16 storage,
+// where a gather and a 3x3-block Cholesky took 2.7.
+constexpr int kFactorTpb = 128;
 
 // Element (r, c) of an 8x8 tile: row-major, the halves of rows with bit 1 set
 // swapped, so that the row-wise and column-wise operand loads of mma.m8n8k4
@@ -105,10 +249,10 @@ __device__ __forceinline__ unsigned short to16<__nv_bfloat16>(double v)
 template <>
 __device__ __forceinline__ unsigned short to16<__half>(double v) { return __half_as_ushort(__float2half_rn((float)v)); }
 
-template <typename TI, int kB>
-__global__ void __launch_bounds__(factor_threads<kB>(), kB == 32 ? 5 : 12) k_domain_invert(FactorArgs a, int dom_offset)
+template <typename TI>
+__global__ void __launch_bounds__(kFactorTpb, 5) k_domain_invert(FactorArgs a, int dom_offset)
 {
-  constexpr int kT = factor_threads<kB>(), kW = kT / 32;
+  constexpr int kB = kBank, kT = kFactorTpb, kW = kT / 32;
   constexpr int kN = 3 * kB, kR = kN / 8;  // rows, tile rows
   constexpr int kTiles = kR * (kR + 1) / 2;
   __shared__ __align__(16) double T[kTiles * 64];
@@ -157,11 +301,6 @@ __global__ void __launch_bounds__(factor_threads<kB>(), kB == 32 ? 5 : 12) k_dom
           if (rp[mid] <= t) lo = mid; else hi = mid;
         }
         if (bc[h] > lo) continue;
-        if (kB == 16 && bc[h] != lo) {
-          // CEMAS16 drops a pair whose slot order runs against its vertex order
-          const int* pm = a.pmr + kB * dom;
-          if (pm[lo] < pm[bc[h]]) continue;
-        }
         br[h] = lo;
 #pragma unroll
         for (int e = 0; e < 9; ++e) v[h][e] = __ldcs(a.val64 + 9 * (size_t)t + e);
@@ -296,93 +435,34 @@ __global__ void __launch_bounds__(factor_threads<kB>(), kB == 32 ? 5 : 12) k_dom
   __syncthreads();
   if (tid == 0 && fail) atomicAdd(a.failed, 1);
 
-  if constexpr (std::is_same<TI, float>::value) {
-    // ---- W^T W, tile (ta, tb) = sum over i >= ta of W_i,ta^T W_i,tb, held as
-    // FP32 until every warp has read W
-    constexpr int kPer = (kTiles + kW - 1) / kW;
-    float m[kPer][2];
-#pragma unroll
-    for (int n = 0; n < kPer; ++n) {
-      const int t = w + n * kW;
-      m[n][0] = m[n][1] = 0.f;
-      if (t >= kTiles) continue;
-      int ta = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
-      while (ta * (ta + 1) / 2 > t) --ta;
-      while ((ta + 1) * (ta + 2) / 2 <= t) ++ta;
-      const int tb = t - ta * (ta + 1) / 2;
-      double c[2] = {0.0, 0.0};
-      for (int i = ta; i < kR; ++i) {
-        const double *A = T + tile_of(i, ta), *B = T + tile_of(i, tb);
-        dmma(c, by_col(A, g, q, 0), by_col(B, g, q, 0));
-        dmma(c, by_col(A, g, q, 1), by_col(B, g, q, 1));
-      }
-      m[n][0] = (float)c[0];
-      m[n][1] = (float)c[1];
-    }
-    __syncthreads();
-    // ---- wrapped diagonals: block (l, (l + d) % kB) at [d][3i + j][l], the
-    // last diagonal for l < kB / 2 only
-    constexpr int kElems = (kB / 2 + 1) * 9 * kB;
-    float* out = reinterpret_cast<float*>(T);
-    static_assert(kElems * sizeof(float) <= sizeof(T) && kElems % 4 == 0, "record fits the tiles");
-    for (int e = tid; e < 9 * kB; e += kT) out[(kB / 2) * 9 * kB + e] = 0.f;
-    __syncthreads();
-#pragma unroll
-    for (int n = 0; n < kPer; ++n) {
-      const int t = w + n * kW;
-      if (t >= kTiles) continue;
-      int ta = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
-      while (ta * (ta + 1) / 2 > t) --ta;
-      while ((ta + 1) * (ta + 2) / 2 <= t) ++ta;
-      const int tb = t - ta * (ta + 1) / 2;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int r = 8 * ta + g, c = 8 * tb + 2 * q + h;
-        if (r < c) continue;  // a diagonal tile's upper half mirrors its lower
-        const int ba = r / 3, i = r % 3, bb = c / 3, j = c % 3, diff = ba - bb;
-        if (diff == 0) {
-          out[(3 * i + j) * kB + ba] = m[n][h];
-          out[(3 * j + i) * kB + ba] = m[n][h];
-        } else if (diff <= kB / 2) {
-          out[(9 * diff + 3 * j + i) * kB + bb] = m[n][h];
-        } else {
-          out[(9 * (kB - diff) + 3 * i + j) * kB + ba] = m[n][h];
-        }
-      }
-    }
-    __syncthreads();
-    float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.inv) + (size_t)dom * kElems);
-    for (int e = tid; e < kElems / 4; e += kT) dst[e] = reinterpret_cast<const float4*>(out)[e];
-  } else {
-    // ---- column scales (largest entry of each column of W) and the scaled
-    // 16-bit tiles, 16 bytes (8 elements of a row) per thread
-    for (int c = tid; c < kN; c += kT) {
-      float m = 0.f;
+  // ---- column scales (largest entry of each column of W) and the scaled
+  // 16-bit tiles, 16 bytes (8 elements of a row) per thread
+  for (int c = tid; c < kN; c += kT) {
+    float m = 0.f;
 #pragma unroll 8
-      for (int r = 0; r < kN; ++r)
-        if (r >= c) m = fmaxf(m, (float)fabs(T[tile_of(r >> 3, c >> 3) + tpos(r & 7, c & 7)]));
-      if (!(m > 0.f) || !isfinite(m)) m = 1.f;
-      colscale[c] = m;
-      a.scale[(size_t)dom * 96 + c] = m;
-    }
-    __syncthreads();
-    uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(a.inv) + (size_t)dom * kInvElems16);
-    for (int e = tid; e < kInvElems16 / 8; e += kT) {
-      const int t16 = e >> 5, r = (e >> 1) & 15, half = (e ^ (r >> 2)) & 1;  // inv16_pos
-      int I = 0;
-      while ((I + 1) * (I + 2) / 2 <= t16) ++I;
-      const int ti = 2 * I + (r >> 3), tj = 2 * (t16 - I * (I + 1) / 2) + half;
-      unsigned u[4] = {0u, 0u, 0u, 0u};
-      if (tj <= ti) {
-        const double* src = T + tile_of(ti, tj);
+    for (int r = 0; r < kN; ++r)
+      if (r >= c) m = fmaxf(m, (float)fabs(T[tile_of(r >> 3, c >> 3) + tpos(r & 7, c & 7)]));
+    if (!(m > 0.f) || !isfinite(m)) m = 1.f;
+    colscale[c] = m;
+    a.scale[(size_t)dom * 96 + c] = m;
+  }
+  __syncthreads();
+  uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(a.inv) + (size_t)dom * kInvElems16);
+  for (int e = tid; e < kInvElems16 / 8; e += kT) {
+    const int t16 = e >> 5, r = (e >> 1) & 15, half = (e ^ (r >> 2)) & 1;  // inv16_pos
+    int I = 0;
+    while ((I + 1) * (I + 2) / 2 <= t16) ++I;
+    const int ti = 2 * I + (r >> 3), tj = 2 * (t16 - I * (I + 1) / 2) + half;
+    unsigned u[4] = {0u, 0u, 0u, 0u};
+    if (tj <= ti) {
+      const double* src = T + tile_of(ti, tj);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const double v = src[tpos(r & 7, k)] / (double)colscale[8 * tj + k];
-          u[k >> 1] |= (unsigned)to16<TI>(v) << (16 * (k & 1));
-        }
+      for (int k = 0; k < 8; ++k) {
+        const double v = src[tpos(r & 7, k)] / (double)colscale[8 * tj + k];
+        u[k >> 1] |= (unsigned)to16<TI>(v) << (16 * (k & 1));
       }
-      dst[e] = make_uint4(u[0], u[1], u[2], u[3]);
     }
+    dst[e] = make_uint4(u[0], u[1], u[2], u[3]);
   }
 }
 
@@ -393,13 +473,13 @@ void factor_domains(maspcg_handle* h, const FactorArgs& a, int g0, int n, int st
 {
   if (n <= 0) return;
   if (h->bank == 16)
-    k_domain_invert<float, 16><<<n, factor_threads<16>(), 0, h->stream>>>(a, g0);
+    k_domain_eliminate<16><<<n, 64, 0, h->stream>>>(a, g0);
   else if (storage == MASPCG_INV_FP32)
-    k_domain_invert<float, 32><<<n, factor_threads<32>(), 0, h->stream>>>(a, g0);
+    k_domain_eliminate<32><<<n, 256, 0, h->stream>>>(a, g0);
   else if (storage == MASPCG_INV_BF16)
-    k_domain_invert<__nv_bfloat16, 32><<<n, factor_threads<32>(), 0, h->stream>>>(a, g0);
+    k_domain_invert<__nv_bfloat16><<<n, kFactorTpb, 0, h->stream>>>(a, g0);
   else
-    k_domain_invert<__half, 32><<<n, factor_threads<32>(), 0, h->stream>>>(a, g0);
+    k_domain_invert<__half><<<n, kFactorTpb, 0, h->stream>>>(a, g0);
   MLAUNCHED(h);
 }
 

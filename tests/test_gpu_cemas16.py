@@ -66,7 +66,8 @@ def test_domain_matrices(systems, which):
 
 
 # (dropping reversed pairs or rows leaves some packed and gapped domain
-# matrices indefinite, so their inverses are not compared)
+# matrices indefinite, so the apply with them is not compared; their inverses
+# are, below, where no pivot fails)
 @pytest.mark.parametrize("which", ["sorted", "cube0"])
 def test_inverses_and_apply(systems, which):
     s = systems[which]
@@ -84,6 +85,41 @@ def test_inverses_and_apply(systems, which):
     assert np.array_equal(d, d.transpose(0, 2, 1))
     z_ref = o.precondition(s.b)
     assert np.linalg.norm(z - z_ref) / np.linalg.norm(z_ref) <= 2e-4
+
+
+@pytest.mark.parametrize("which", ["packed", "gapped"])
+def test_inverses_of_partitions_that_lose_entries(systems, which):
+    """The gapped partition's coarse diagonal blocks are not symmetric (its rows
+    enter one triangle only), and the inverse is that of the matrix as it is.
+    Blocks up to eight columns from the diagonal: the others are stored as the
+    mirror of the inverse's lower triangle.  1e-5 of the largest entry: FP32
+    rounding, and the 1e-13 by which the sums may differ at condition numbers of
+    1e6; the inverse of one triangle alone is 4e-4 to 1e-2 off."""
+    s = systems[which]
+    p64, i32 = _oracle(s).domains()
+    with MasPcg.from_system(s, preconditioner="cemas16") as m:
+        gi, info = m.domain_inverses(), m.info()
+    A = np.zeros((len(p64), 48, 48))
+    q = 0
+    for a in range(16):
+        for b in range(a, 16):
+            B = p64[:, q].reshape(-1, 3, 3).transpose(0, 2, 1)
+            A[:, 3 * b:3 * b + 3, 3 * a:3 * a + 3] = B.transpose(0, 2, 1)
+            A[:, 3 * a:3 * a + 3, 3 * b:3 * b + 3] = B
+            q += 1
+    d = np.arange(48)
+    diagonal = A[:, d, d]
+    A[:, d, d] = np.where(diagonal == 0, 1.0, diagonal)
+    ok = np.ones(len(A), bool)
+    for j in range(48):  # the pivots of an elimination without exchanges
+        ok &= A[:, j, j] > 1e-6 * np.abs(A).max(axis=(1, 2))
+        p = np.where(ok, A[:, j, j], 1.0)
+        A[ok, j + 1:] -= (A[ok, j + 1:, j] / p[ok, None])[:, :, None] * A[ok, j, None]
+    assert info["failed_domains"] <= np.count_nonzero(~ok) and np.count_nonzero(ok) > 0.9 * len(ok)
+    assert np.count_nonzero(ok[len(s.part_map_real) // 16:]) >= 5
+    near = [b - a <= 8 for a in range(16) for b in range(a, 16)]
+    scale = np.abs(i32[ok]).max(axis=(1, 2))[:, None, None]
+    assert np.max((np.abs(gi[ok] - i32[ok]) / scale)[:, near]) <= 1e-5
 
 
 @pytest.mark.parametrize("gate", ["rz", "euclid"])
