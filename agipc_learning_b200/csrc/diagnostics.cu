@@ -171,11 +171,7 @@ void check_local_matrices(maspcg_handle* h, int count, int bank, const double* p
   cudaStream_t st = h->stream;
   if (bank == 32) {
     constexpr int bytes = 2 * 96 * 96 * sizeof(double);
-    static bool cfg = false;
-    if (!cfg) {
-      MCK(cudaFuncSetAttribute(k_local_checks<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-      cfg = true;
-    }
+    allow_smem(h, k_local_checks<32>, bytes);
     k_local_checks<32><<<count, kDiagTpb, bytes, st>>>(packed64_dev, inverse32_dev, results_dev);
   } else {
     constexpr int bytes = 2 * 48 * 48 * sizeof(double);

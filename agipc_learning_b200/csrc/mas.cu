@@ -1520,11 +1520,7 @@ void launch_apply_tma(maspcg_handle* h, const ApplyArgs& a, const Tv* r, Tv* z, 
 {
   constexpr int bytes = kApplyWarps * (kBuf * kRecBytes16 + kApplyScratch);
   auto kern = k_apply_tma<TI, Tv, Tacc, kBuf, kFused, kLevel1>;
-  static bool configured = false;
-  if (!configured) {
-    MCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    configured = true;
-  }
+  allow_smem(h, kern, bytes);
   launch_pdl(h, kern, dim3(grid), dim3(kApplyWarps * 32), bytes, a, r, z, partial, part_base, total_parts, mode, s,
              g_end, h->failed.get() + 4, coarse_add, pair, fa, partial_rr);
 }
@@ -1592,9 +1588,7 @@ void launch_coarse(maspcg_handle* h, cudaStream_t st, const ApplyArgs& a, const 
     launch_pdl_on(h, st, k_restrict1<Tv, kB, kFused>, dim3(ceil_div(h->c0, kTpb)), dim3(kTpb), 0, a, r, s, fa);
   if (from_level >= a.lv.levelnum) return;
   constexpr int bytes = (kCoarseStage + 2 * 3 * kCoarseOnChip) * sizeof(float);
-  static bool configured = false;
-  if (!configured) MCK(cudaFuncSetAttribute(k_coarse_levels<TI, kB>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  configured = true;
+  allow_smem(h, k_coarse_levels<TI, kB>, bytes);
   launch_pdl_on(h, st, k_coarse_levels<TI, kB>, dim3(a.lv.domains - a.lv.dom_begin[from_level]),
                 dim3(coarse_threads<TI, kB>()), bytes, coarse_levels_args(h), s, mode, pair, h->chain_dot.get());
 }

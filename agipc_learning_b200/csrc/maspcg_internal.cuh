@@ -20,6 +20,7 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <utility>
@@ -197,6 +198,7 @@ struct maspcg_handle {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   int device = 0;
   int sm_count = 148;
+  std::vector<const void*> wide_smem;  // kernels let beyond 48 KB of dynamic shared memory on this device
   std::string last_error;
 
   // ---- graph (set_graph)
@@ -451,6 +453,18 @@ inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 // Without the launch attribute both instructions are no-ops.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Lets a kernel take `bytes` of dynamic shared memory, above the 48 KB that need
+// no leave.  The limit is the device's own, so the mark is kept by the handle,
+// which belongs to one device, and not by the process.
+template <typename... KArgs>
+void allow_smem(maspcg_handle* h, void (*kernel)(KArgs...), int bytes)
+{
+  const void* k = reinterpret_cast<const void*>(kernel);
+  if (std::find(h->wide_smem.begin(), h->wide_smem.end(), k) != h->wide_smem.end()) return;
+  MCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  h->wide_smem.push_back(k);
+}
 
 template <typename... KArgs, typename... Args>
 void launch_pdl_on(maspcg_handle* h, cudaStream_t stream, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,

@@ -73,3 +73,17 @@ def test_create_without_device_fails_cleanly(lib):
     h = ctypes.c_void_p()
     assert lib.maspcg_create(None, ctypes.byref(h)) == N.ERR_NO_DEVICE
     assert not h.value
+
+
+def test_shared_memory_limits_are_set_per_handle():
+    """cudaFuncSetAttribute acts on the current device, and a process may hold
+    handles on several: the mark that a kernel's limit is set is the handle's, so
+    no launch may keep one of its own (a function-local static)."""
+    csrc = os.path.join(ROOT, "agipc_learning_b200", "csrc")
+    for name in sorted(os.listdir(csrc)):
+        text = open(os.path.join(csrc, name)).read()
+        calls = [m.start() for m in re.finditer(r"cudaFuncSetAttribute\(", text)]
+        if name == "maspcg_internal.cuh":
+            assert len(calls) == 1 and text.rindex("void allow_smem(", 0, calls[0]) < calls[0]
+        else:
+            assert not calls, name

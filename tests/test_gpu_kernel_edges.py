@@ -271,3 +271,19 @@ def test_rows_around_the_bucket_limits(long_row):
     ref = oracle.sym_spmv(1.0, v, r, c, x)
     mag = oracle.sym_spmv(1.0, np.abs(v), r, c, np.abs(x))
     assert np.all(np.abs(y - ref) <= 3 * 3000 * np.finfo(np.float64).eps * mag + 1e-300)
+
+
+@pytest.mark.parametrize("inverse", ["fp32", "bf16"])
+def test_handles_on_two_devices(inverse):
+    """A handle on a second GPU, after one on the first: a kernel's limit of
+    shared memory is a device's own.  Solves, and the local checks."""
+    import torch
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    s = synth.cube_system(9, E=1e5, seed=1)
+    x = []
+    for device in (0, 1):
+        with torch.cuda.device(device), MasPcg.from_system(s, precision="mixed", inverse=inverse, gate="euclid") as m:
+            x.append(m.solve(s.b)[0])
+            assert m.local_diagnostics()["matrix_count"] > 0
+    assert np.linalg.norm(x[0] - x[1]) <= 1e-6 * np.linalg.norm(x[0])
