@@ -278,11 +278,14 @@ __global__ void __launch_bounds__(kFemTpb, 3) k_fem_snk1(int ntet, const unsigne
   const double ev2 = rr * (2.0 * I3 - 1.0) - u;
   double A[6] = {u + rr * S[1] * S[1] * S[2] * S[2], u + rr * S[0] * S[0] * S[2] * S[2],
                  u + rr * S[0] * S[0] * S[1] * S[1], ev2 * S[2], ev2 * S[1], ev2 * S[0]};  // 00 11 22 01 02 12
-  // positive leading minors: the projection changes nothing (most tets);
-  // otherwise the eigenvalues below zero are cut off
+  // leading minors positive beyond their own rounding (some 1e-15 of the trace's
+  // powers): the projection changes nothing (most tets; the determinant is 1e-2 of
+  // the trace cubed at a Poisson ratio of 0.45, 1e-7 at 0.4999).  Otherwise the
+  // eigenvalues below zero are cut off
   const double m01 = A[0] * A[1] - A[3] * A[3];
   const double det = A[2] * m01 - A[0] * A[5] * A[5] - A[1] * A[4] * A[4] + 2.0 * A[3] * A[4] * A[5];
-  if (!(A[0] > 0.0 && m01 > 0.0 && det > 0.0)) {
+  const double tr = A[0] + A[1] + A[2];
+  if (!(A[0] > 1e-12 * tr && m01 > 1e-12 * tr * tr && det > 1e-12 * tr * tr * tr)) {
     const double f = pow2_scale(fmax(fabs(A[0]), fmax(fabs(A[1]), fmax(fabs(A[2]), fmax(fabs(A[3]),
                                                                     fmax(fabs(A[4]), fabs(A[5])))))));
     double d[6], W[9];

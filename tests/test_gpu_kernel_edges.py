@@ -69,6 +69,36 @@ def test_element_kernel_degenerate_tets():
             assert np.abs(V1 - V0).max() <= 1e-9 * np.abs(V0).max(), F
 
 
+def test_element_kernel_nearly_singular_projection():
+    """Tets whose scaling Hessian has two eigenvalues around 1e-9 of the third and
+    of opposite signs, so that its determinant is lost in rounding: the negative
+    one is projected out all the same (1e-9 of each tet's largest entry)."""
+    rng = np.random.default_rng(0)
+    n = 200000
+    S = 10.0 ** rng.uniform(-0.6, 0.6, (n, 3))
+    u = 10.0 ** rng.uniform(-9.5, -6.5, n)
+    S *= ((1 + u * (1 + rng.uniform(-8, 8, n))) / S.prod(axis=1))[:, None] ** (1 / 3)
+    S = -np.sort(-S, axis=1)
+    J = S.prod(axis=1)
+    A = ((2 * J - 1 - u) / J)[:, None, None] * J[:, None, None] ** 2 / (S[:, :, None] * S[:, None, :])
+    d = np.arange(3)
+    A[:, d, d] = u[:, None] + (J[:, None] / S) ** 2
+    w = np.linalg.eigvalsh(A) / np.abs(A).max(axis=(1, 2))[:, None]
+    S, u = (a[(w[:, 0] < -2e-9) & (w[:, 1] > 0) & (w[:, 1] < 2e-9)] for a in (S, u))
+    n = len(u)
+    assert n > 100
+    Q = np.linalg.qr(rng.standard_normal((2, n, 3, 3)))[0]
+    F = (Q[0] * S[:, None, :]) @ Q[1].transpose(0, 2, 1)
+    F *= np.sign(np.linalg.det(F))[:, None, None]
+    x = np.concatenate([np.zeros((n, 1, 3)), F.transpose(0, 2, 1)], axis=1).reshape(-1, 3)
+    tets = np.arange(4 * n, dtype=np.int32).reshape(n, 4)
+    Di, one = np.tile(np.eye(3).reshape(1, 9), (n, 1)), np.ones(n)
+    V0 = oracle.fem_snk1(tets, x, Di, one, u, one, 1.0)[3].reshape(n, 90)
+    with MasPcg() as m:
+        V1 = m.fem_snk1(tets, x, Di, one, u, one, 1.0)[3].reshape(n, 90)
+    assert np.all(np.abs(V1 - V0).max(axis=1) <= 1e-9 * np.abs(V0).max(axis=1))
+
+
 @pytest.mark.parametrize("n,run", [(2, 1), (31, 2), (255, 3), (257, 4), (2303, 5), (2305, 9)])
 def test_merge_run_lengths(n, run):
     """Runs around the four-ahead fetch and element counts around a CTA:
