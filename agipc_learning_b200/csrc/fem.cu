@@ -155,9 +155,9 @@ __device__ __forceinline__ void signed_svd3(const double F[9], double U[9], doub
 }
 
 // The warp's 32 x 9 values (a block of each tet, lane by lane in stage) to
-// out + 90 lane: runs of 72 bytes, nine coalesced stores.
+// out + 90 lane for the tets of the mask: runs of 72 bytes, nine coalesced stores.
 __device__ __forceinline__ void store_blocks(double* stage, const double K[9], bool swap, double* out, int lane,
-                                             int tets)
+                                             unsigned tets)
 {
   double* mine = stage + 9 * lane;  // Eigen column-major; a swapped block is transposed
 #pragma unroll
@@ -168,7 +168,7 @@ __device__ __forceinline__ void store_blocks(double* stage, const double K[9], b
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
     const int e = lane + 32 * k, t = e / 9;
-    if (t < tets) __stcs(out + 90 * (size_t)t + e % 9, stage[e]);
+    if ((tets >> t) & 1u) __stcs(out + 90 * (size_t)t + e % 9, stage[e]);
   }
   __syncwarp();
 }
@@ -186,7 +186,6 @@ __global__ void __launch_bounds__(kFemTpb, 3) k_fem_snk1(int ntet, const unsigne
   double* stage = stage_s[threadIdx.x >> 5];
   const int first = blockIdx.x * blockDim.x + (threadIdx.x & ~31);
   if (first >= ntet) return;  // whole warp
-  const int tets_here = min(32, ntet - first);
   // lanes past the end repeat the last tet without writing
   const int t = min(first + lane, ntet - 1);
   const bool own = first + lane < ntet;
@@ -194,10 +193,11 @@ __global__ void __launch_bounds__(kFemTpb, 3) k_fem_snk1(int ntet, const unsigne
   const bool fits = v[0] < (unsigned)nverts && v[1] < (unsigned)nverts && v[2] < (unsigned)nverts &&
                     v[3] < (unsigned)nverts;
   if (!fits) {
-    atomicExch(bad, 1);  // the call reports the error; the tet's outputs are unspecified
+    atomicExch(bad, 1);  // the tet is skipped; the call reports the error
 #pragma unroll
     for (int a = 0; a < 4; ++a) v[a] = 0;
   }
+  const unsigned tets_here = __ballot_sync(kFull, own && fits);
   double Di[9];  // row-major Dm^-1
 #pragma unroll
   for (int e = 0; e < 9; ++e) Di[e] = dm_inv[9 * (size_t)t + e];
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(kFemTpb, 3) k_fem_snk1(int ntet, const unsigne
       int* out = (which ? cols : rows) + 10 * (size_t)first;
 #pragma unroll
       for (int k = 0; k < 10; ++k)
-        if (lane + 32 * k < 10 * tets_here) out[lane + 32 * k] = st[lane + 32 * k];
+        if ((tets_here >> ((lane + 32 * k) / 10)) & 1u) out[lane + 32 * k] = st[lane + 32 * k];
       __syncwarp();
     }
   }

@@ -69,6 +69,36 @@ def test_element_kernel_degenerate_tets():
             assert np.abs(V1 - V0).max() <= 1e-9 * np.abs(V0).max(), F
 
 
+def test_element_kernel_skips_bad_tets():
+    """A vertex id outside the mesh is refused, the outputs of that tet's own
+    slots are left alone and the other tets' are written as without it."""
+    import torch
+    X, tets = synth.box_mesh(4, 4, 3, 0.01)
+    nt = 45
+    tets = np.ascontiguousarray(tets[:nt], np.int32)
+    bad = [0, 31, 40]
+    Di, vol, u, r = oracle.fem_rest_data(tets, X, np.full(nt, 1e5), 0.45)
+    _, R0, C0, V0 = oracle.fem_snk1(tets, X, Di, vol, u, r, 0.01)
+    tets[bad, [0, 3, 1]] = len(X)
+    D = lambda a, t: torch.from_numpy(np.ascontiguousarray(a, t)).cuda()  # noqa: E731
+    rows = torch.full((nt, 10), -7, dtype=torch.int32, device="cuda")
+    cols, vals = rows.clone(), torch.full((nt, 90), 5.0, dtype=torch.float64, device="cuda")
+    grad = torch.zeros(X.size, dtype=torch.float64, device="cuda")
+    a = [D(tets, np.int32), D(X, np.float64), D(Di, np.float64), D(vol, np.float64), D(u, np.float64), D(r, np.float64)]
+    p = [t.data_ptr() for t in a]
+    torch.cuda.synchronize()
+    with MasPcg() as m, pytest.raises(RuntimeError, match="vertex id out of range"):
+        N.check(m.lib.maspcg_fem_snk1_gradient_hessian(m.h, nt, p[0], len(X), p[1], p[2], p[3], p[4], p[5], 0.01, 0,
+                                                       grad.data_ptr(), rows.data_ptr(), cols.data_ptr(),
+                                                       vals.data_ptr()), m.h)
+    good = np.setdiff1d(np.arange(nt), bad)
+    R, C, V = rows.cpu().numpy(), cols.cpu().numpy(), vals.cpu().numpy()
+    assert np.all(R[bad] == -7) and np.all(C[bad] == -7) and np.all(V[bad] == 5.0)
+    assert np.array_equal(R[good], R0.reshape(nt, 10)[good]) and np.array_equal(C[good], C0.reshape(nt, 10)[good])
+    V0 = V0.reshape(nt, 90)
+    assert np.all(np.abs(V - V0)[good].max(axis=1) <= 1e-9 * np.abs(V0[good]).max(axis=1))
+
+
 def test_element_kernel_nearly_singular_projection():
     """Tets whose scaling Hessian has two eigenvalues around 1e-9 of the third and
     of opposite signs, so that its determinant is lost in rounding: the negative
