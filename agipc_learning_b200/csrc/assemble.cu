@@ -29,33 +29,6 @@ namespace {
 
 constexpr int kAsmTpb = 256;
 
-// Largest row and column index (for the key width), and a flag for
-// negative indices: a grid-stride pass with one set of atomics per CTA (an
-// atomic pair per warp, all on two addresses, took longer than the sort).
-__global__ void __launch_bounds__(kAsmTpb) k_conv_range(const int* __restrict__ rows, const int* __restrict__ cols,
-                                                       int n, int* flags)
-{
-  __shared__ unsigned most[2][kAsmTpb / 32];
-  unsigned r = 0, c = 0;
-  bool negative = false;
-  for (int i = blockIdx.x * kAsmTpb + threadIdx.x; i < n; i += gridDim.x * kAsmTpb) {
-    const int ri = rows[i], ci = cols[i];
-    negative |= ri < 0 || ci < 0;
-    r = max(r, (unsigned)max(ri, 0));
-    c = max(c, (unsigned)max(ci, 0));
-  }
-  r = __reduce_max_sync(0xffffffffu, r);
-  c = __reduce_max_sync(0xffffffffu, c);
-  if ((threadIdx.x & 31) == 0) most[0][threadIdx.x >> 5] = r, most[1][threadIdx.x >> 5] = c;
-  negative = __syncthreads_or(negative);
-  if (threadIdx.x < 2) {
-    unsigned v = 0;
-    for (int w = 0; w < kAsmTpb / 32; ++w) v = max(v, most[threadIdx.x][w]);
-    atomicMax(flags + 1 + threadIdx.x, (int)v);
-  }
-  if (threadIdx.x == 0 && negative) atomicExch(flags, 1);
-}
-
 // Key (row << col_bits) + col: the order of (row << 32) + col in as few bits
 // as the indices need, so the radix sort runs only the passes it must.
 __global__ void k_conv_keys(const int* __restrict__ rows, const int* __restrict__ cols, int n, int col_bits,
@@ -152,30 +125,23 @@ MergedKeys merge_keys(maspcg_handle* h, const int* rows, const int* cols, int n)
   MergedKeys out{};
   if (n <= 0) return out;
   cudaStream_t st = h->stream;
-  h->asm_keys.resize(2 * (size_t)n);
+  TripletRange top{};
+  if (row_sort_triplets(h, rows, cols, n, top, out)) return out;
+  unsigned long long* k0 = h->asm_keys.get();  // 2n at least
+  unsigned long long* k1 = k0 + n;
   h->asm_idx.resize(2 * (size_t)n);
   h->asm_flags.resize(2 * (size_t)n + 4);
-  unsigned long long* k0 = h->asm_keys.get();
-  unsigned long long* k1 = k0 + n;
   int* i0 = h->asm_idx.get();
   int* i1 = i0 + n;
   int* heads = h->asm_flags.get();
   int* pos = heads + n;
-  int* flags = pos + n;  // negative index, max row, max col
-  MCK(cudaMemsetAsync(flags, 0, 3 * sizeof(int), st));
   const int grid = ceil_div(n, kAsmTpb);
-  k_conv_range<<<std::min(grid, 8 * h->sm_count), kAsmTpb, 0, st>>>(rows, cols, n, flags); MLAUNCHED(h);
-  int fl[3] = {0, 0, 0};
-  MCK(cudaMemcpyAsync(fl, flags, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
-  MCK(cudaStreamSynchronize(st));
-  MREQ(fl[0] == 0, MASPCG_ERR_INVALID_ARGUMENT, "negative row or column index");
   auto bits = [](unsigned v) {
     int b = 1;
     while (b < 32 && (v >> b) != 0u) ++b;
     return b;
   };
-  if (row_sort_triplets(h, rows, cols, n, fl[1], out)) return out;
-  const int col_bits = bits((unsigned)fl[2]), key_bits = col_bits + bits((unsigned)fl[1]);
+  const int col_bits = bits((unsigned)top.col), key_bits = col_bits + bits((unsigned)top.row);
   k_conv_keys<<<grid, kAsmTpb, 0, st>>>(rows, cols, n, col_bits, k0, i0); MLAUNCHED(h);
   size_t need = 0;
   MCK(cub::DeviceRadixSort::SortPairs(nullptr, need, k0, k1, i0, i1, n, 0, key_bits, st));

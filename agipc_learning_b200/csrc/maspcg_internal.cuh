@@ -343,11 +343,15 @@ void modulus_gradient(maspcg_handle* h, const int* rows, const int* cols, const 
 
 // rowsort.cu: the merge order by row buckets; false leaves it to a radix sort.
 // row_sort_matrix fills rowptr, colidx, seg_start, kv_sorted, m_valid and nnzb
-// of the symmetric structure; row_sort_triplets the order of n triplets with
-// rows up to last_row.
+// of the symmetric structure; row_sort_triplets the order of n triplets, and in
+// any case the largest row and column (asm_keys then holds 2n at least).  Both
+// refuse indices out of range.
 struct MergedKeys;
+struct TripletRange {
+  int row, col;
+};
 bool row_sort_matrix(maspcg_handle* h, const int* rows, const int* cols, int n);
-bool row_sort_triplets(maspcg_handle* h, const int* rows, const int* cols, int n, int last_row, MergedKeys& out);
+bool row_sort_triplets(maspcg_handle* h, const int* rows, const int* cols, int n, TripletRange& range, MergedKeys& out);
 
 // assemble.cu (device pointers; returns the unique count / the type counts)
 // The triplets' order and runs by (row, col): entries perm[start[u]] ..

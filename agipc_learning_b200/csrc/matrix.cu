@@ -73,6 +73,15 @@ __global__ void k_heads(const unsigned long long* __restrict__ keys, int m, int*
   head[i] = (k != kSentinel && (i == 0 || k != keys[i - 1])) ? 1 : 0;
 }
 
+// Block count, indices out of range and sentinels of the sorted structure in one
+// place: one copy to the host (each waits for the stream) where there were three.
+__global__ void k_structure_ends(const int* last_head, const int* last_index, const int* flags, int* ends)
+{
+  ends[0] = *last_head + *last_index;
+  ends[1] = flags[0];
+  ends[2] = flags[2];
+}
+
 __global__ void k_fill_structure(const unsigned long long* __restrict__ keys, const int* __restrict__ head,
                                  const int* __restrict__ uidx, int m, int bits, int* colidx, int* seg_start,
                                  int* row_count)
@@ -328,14 +337,16 @@ void radix_sort_matrix(maspcg_handle* h, const int* rows, const int* cols, int n
   // unique index = exclusive scan of heads (reuse kv as output)
   tb = h->cub_tmp.cap;
   MCK(cub::DeviceScan::ExclusiveSum(h->cub_tmp.get(), tb, h->seg_head.get(), h->kv.get(), m, st));
-  int tail[2] = {0, 0}, flags[3] = {0, 0, 0};
-  MCK(cudaMemcpyAsync(&tail[0], h->kv.get() + (m - 1), sizeof(int), cudaMemcpyDeviceToHost, st));
-  MCK(cudaMemcpyAsync(&tail[1], h->seg_head.get() + (m - 1), sizeof(int), cudaMemcpyDeviceToHost, st));
-  MCK(cudaMemcpyAsync(flags, h->failed.get(), 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  int* ends = h->failed.get() + 4;
+  k_structure_ends<<<1, 1, 0, st>>>(h->seg_head.get() + (m - 1), h->kv.get() + (m - 1), h->failed.get(), ends);
+  MLAUNCHED(h);
+  int e[3] = {0, 0, 0};
+  MCK(cudaMemcpyAsync(e, ends, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
   MCK(cudaStreamSynchronize(st));
-  MREQ(flags[0] == 0, MASPCG_ERR_INVALID_ARGUMENT, "matrix block index out of range");
-  const int nnzb = tail[0] + tail[1];
-  const int m_valid = m - flags[2];  // sentinels (one per diagonal input block) sort last
+  MCK(cudaMemsetAsync(ends, 0, 3 * sizeof(int), st));
+  MREQ(e[1] == 0, MASPCG_ERR_INVALID_ARGUMENT, "matrix block index out of range");
+  const int nnzb = e[0];
+  const int m_valid = m - e[2];  // sentinels (one per diagonal input block) sort last
   h->m_valid = m_valid;
   h->nnzb = nnzb;
   h->colidx.resize(nnzb, 4);  // 16-byte tail for TMA bulk copies
@@ -377,7 +388,7 @@ void build_internal_matrix(maspcg_handle* h, const double* vals, const int* rows
   h->seg_start.resize(m + 1);
   h->failed.resize(8);
   MCK(cudaMemsetAsync(h->failed.get(), 0, sizeof(int) * 8, st));
-  h->row_count.resize(nb_int + 1);
+  h->row_count.resize((size_t)nb_int + 5);
   h->rowptr.resize(nb_int + 1);
   if (!row_sort_matrix(h, rows, cols, n)) radix_sort_matrix(h, rows, cols, n);
   const int nnzb = h->nnzb;

@@ -333,6 +333,55 @@ def test_rows_around_the_bucket_limits(long_row):
     assert np.all(np.abs(y - ref) <= 3 * 3000 * np.finfo(np.float64).eps * mag + 1e-300)
 
 
+@pytest.mark.parametrize("last_row", [65597, 65598, 65599, 2 ** 31 - 2])
+def test_rows_around_the_bucket_rule(last_row):
+    """1,000 triplets in rows up to the last that buckets are kept for (1,000 / 16
+    + 65,536 of them), the next two and the largest index: the merge bit-exact,
+    and the product of a matrix of as many rows."""
+    rng = np.random.default_rng(last_row % 1000)
+    n = 1000
+    r = np.concatenate([rng.integers(0, 60000, n - 2), [last_row, last_row]]).astype(np.int32)
+    c = np.concatenate([rng.integers(60000, 60100, n - 2), [last_row, last_row]]).astype(np.int32)
+    r[:300] = r[300:600]  # some repeats
+    c[:300] = c[300:600]
+    o = rng.permutation(n)
+    r, c, v = r[o], c[o], rng.standard_normal((n, 9))
+    ro, co, vo = oracle.convert_triplets(r, c, v)
+    with MasPcg(preconditioner="none", precision="reference") as m:
+        rg, cg, vg = m.convert_bcoo(r, c, v)
+        assert np.array_equal(rg, ro) and np.array_equal(cg, co) and np.array_equal(vg, vo)
+        if last_row > 70000:
+            return
+        nb = last_row + 64  # twice the entries: rows around 2,000 / 16 + 65,536
+        x = rng.standard_normal(3 * nb)
+        m.set_matrix(v, r, c, nb)
+        y = m.spmv(x)
+    ref, mag = oracle.sym_spmv(1.0, v, r, c, x), oracle.sym_spmv(1.0, np.abs(v), r, c, np.abs(x))
+    assert np.all(np.abs(y - ref) <= 3 * n * np.finfo(np.float64).eps * mag)
+
+
+@pytest.mark.parametrize("where", ["spread", "last"])
+def test_long_row_among_many_triplets(where):
+    """A row of 5,000 among 700,000 triplets, met in the first or in a later round
+    of the counting pass: the merge bit-exact, the product to the FP64 bound."""
+    rng = np.random.default_rng(11)
+    n, nb = 700000, 60000
+    r = rng.integers(0, nb, n)
+    at = rng.permutation(n)[:5000] if where == "spread" else np.arange(n - 5000, n)
+    r[at] = 77
+    c = np.maximum(r, rng.integers(0, nb, n))
+    r, c, v = r.astype(np.int32), c.astype(np.int32), rng.standard_normal((n, 9))
+    x = rng.standard_normal(3 * nb)
+    ro, co, vo = oracle.convert_triplets(r, c, v)
+    with MasPcg(preconditioner="none", precision="reference") as m:
+        rg, cg, vg = m.convert_bcoo(r, c, v)
+        m.set_matrix(v, r, c, nb)
+        y = m.spmv(x)
+    assert np.array_equal(rg, ro) and np.array_equal(cg, co) and np.array_equal(vg, vo)
+    ref, mag = oracle.sym_spmv(1.0, v, r, c, x), oracle.sym_spmv(1.0, np.abs(v), r, c, np.abs(x))
+    assert np.all(np.abs(y - ref) <= 3 * 5100 * np.finfo(np.float64).eps * mag)
+
+
 @pytest.mark.parametrize("inverse", ["fp32", "bf16"])
 def test_handles_on_two_devices(inverse):
     """A handle on a second GPU, after one on the first: a kernel's limit of
