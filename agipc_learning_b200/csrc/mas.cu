@@ -48,15 +48,6 @@ __global__ void k_member_keys(const int* __restrict__ cmap, int c0, int count, u
   vals[s] = s;
 }
 
-__global__ void k_member_offsets(const unsigned* __restrict__ keys, int nreal, int count, int* off)
-{
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= nreal) return;
-  const unsigned k = keys[p];
-  if (p == 0 || keys[p - 1] != k) off[k] = p;
-  if (p == nreal - 1) off[count] = nreal;
-}
-
 template <int kB>
 __device__ __forceinline__ int pkb(int a, int b) { return kB * a - a * (a + 1) / 2 + b; }
 
@@ -476,9 +467,7 @@ constexpr int kDirectSmem16 = (kApplyTpb / 32) * (kRecBytes16 + kApplyScratch);
 // more and wider (6,912 level-1 nodes below one CTA at 110,592 rows), and the
 // kernel per level stays ahead of this form (75.5 against 82.9 us per iteration).
 
-// The children of every level-l node: they lie in one bank of level l - 1 (kB
-// nodes), so a node keeps that bank and the bits of its children's lanes.
-template <int kB>
+// The children of every level-l node: they lie in one bank of level l - 1, so a node keeps that bank and the bits of its children's lanes.
 __global__ void k_children(const int* __restrict__ going_next, int begin_prev, int count_prev, int begin_next,
                            int* child_bank, unsigned* child_mask)
 {
@@ -488,8 +477,8 @@ __global__ void k_children(const int* __restrict__ going_next, int begin_prev, i
   const int key = t < count_prev ? going_next[begin_prev + t] - begin_next : -1;
   const unsigned grp = __match_any_sync(kFull, key);
   if (key < 0 || __ffs(grp) - 1 != lane) return;
-  child_bank[key] = t / kB;
-  child_mask[key] = kB == 32 ? grp : grp >> (lane & 16);
+  child_bank[key] = t / kBank;
+  child_mask[key] = grp;
 }
 
 struct CoarseLevels {
@@ -530,18 +519,17 @@ __device__ __forceinline__ int domain_level(const LevelInfo& lv, int g)
 
 // The nodes of every level below a coarse domain of level l >= 2, down to level
 // 1 (whole banks: a span may hold a few nodes of a neighbouring domain).
-template <int kB>
 __global__ void k_coarse_spans(CoarseLevels a)
 {
   const int g = a.lv.dom_begin[1] + blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= a.lv.domains) return;
   const int l = domain_level(a.lv, g);
   int2* span = a.span + (size_t)(g - a.lv.dom_begin[1]) * kMaxLevels;
-  int lo = kB * g - a.lv.begin[l], hi = min(lo + kB, a.lv.count[l]);
+  int lo = kBank * g - a.lv.begin[l], hi = min(lo + kBank, a.lv.count[l]);
   span[l] = make_int2(lo, hi);
   for (int m = l; m >= 2; --m) {
-    lo = kB * a.child_bank[m][lo];
-    hi = min(a.lv.count[m - 1], kB * (a.child_bank[m][hi - 1] + 1));
+    lo = kBank * a.child_bank[m][lo];
+    hi = min(a.lv.count[m - 1], kBank * (a.child_bank[m][hi - 1] + 1));
     span[m - 1] = make_int2(lo, hi);
   }
 }
@@ -549,8 +537,8 @@ __global__ void k_coarse_spans(CoarseLevels a)
 // Threads of a coarse domain's CTA: one 16-byte load per thread fetches a 16-bit
 // record (21 tiles of 16x16, six warps apply them), a thread per block of the
 // wrapped diagonals of an FP32 one.
-template <typename TI, int kB>
-constexpr int coarse_threads() { return sizeof(TI) == 2 ? 32 * kTiles16 : kDiags * kB; }
+template <typename TI>
+constexpr int coarse_threads() { return sizeof(TI) == 2 ? 32 * kTiles16 : kDiags * kBank; }
 
 // One coarse domain per CTA: R of its nodes, then Z = M R with the whole record
 // on the chip, loaded before R is needed.  Latency is all that counts here
@@ -563,13 +551,12 @@ constexpr int coarse_threads() { return sizeof(TI) == 2 ? 32 * kTiles16 : kDiags
 // to the p update; this kernel then also sums r.z of the coarse levels, the
 // sum over domains of R.Z (= r . P Z), and completes r.z with the level-0
 // part (rz_part_done, mode as in rz_update).
-template <typename TI, int kB>
-__global__ void __launch_bounds__(coarse_threads<TI, kB>(), 2) k_coarse_levels(CoarseLevels a, PcgScalars* s, int mode,
+template <typename TI>
+__global__ void __launch_bounds__(coarse_threads<TI>(), 2) k_coarse_levels(CoarseLevels a, PcgScalars* s, int mode,
                                                                           int pair, double* dots)
 {
-  constexpr int kT = coarse_threads<TI, kB>(), kN = 3 * kB;
+  constexpr int kT = coarse_threads<TI>(), kN = 3 * kBank;
   constexpr bool kTiled = sizeof(TI) == 2;
-  constexpr int kD = kB / 2 + 1;  // wrapped diagonals of an FP32 record
   // dynamic: R of the levels below (two of them), then R of a level on the way
   // up (the partial products afterwards)
   extern __shared__ __align__(16) float coarse_smem[];
@@ -577,21 +564,21 @@ __global__ void __launch_bounds__(coarse_threads<TI, kB>(), 2) k_coarse_levels(C
   __shared__ float xs[kN], vs[kN], norm[2];
   __shared__ __align__(4) unsigned short part[kTiled ? 3 * kPartStride : 1];
   float* p1 = stage;
-  float* p2 = stage + kD * kN;
+  float* p2 = stage + kDiags * kN;
   static_assert(2 * kDiags * 3 * kBank <= kCoarseStage, "partial products share the stage");
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
   const int g = a.lv.domains - 1 - blockIdx.x;  // the top levels, with most below them, start first
   // the record does not change during a solve: it is fetched before the wait
   uint4 rec;
   float sc = 1.f, B[9];
-  const int d = tid / kB, ln = tid % kB;
+  const int d = tid / kBank, ln = tid % kBank;
   if constexpr (kTiled) {
     rec = __ldg(reinterpret_cast<const uint4*>(a.inv) + (size_t)g * (kRecBytes16 / 16) + tid);
     if (tid < kN) sc = __ldg(a.scale + (size_t)g * 96 + tid);
-  } else if (d < kD) {
-    const float* src = reinterpret_cast<const float*>(a.inv) + (size_t)g * (kD * 9 * kB);
+  } else if (d < kDiags) {
+    const float* src = reinterpret_cast<const float*>(a.inv) + (size_t)g * (kDiags * 9 * kBank);
 #pragma unroll
-    for (int e = 0; e < 9; ++e) B[e] = __ldg(src + (d * 9 + e) * kB + ln);
+    for (int e = 0; e < 9; ++e) B[e] = __ldg(src + (d * 9 + e) * kBank + ln);
   }
   pdl_wait();
   if (s && s->status != MASPCG_SOLVE_RUNNING) return;  // uniform: nothing changes the status meanwhile
@@ -613,8 +600,8 @@ __global__ void __launch_bounds__(coarse_threads<TI, kB>(), 2) k_coarse_levels(C
     auto parents = [&](int m, int bank) {
       const int* next = a.going_next + a.lv.begin[m - 1];
       Parents t;
-      t.first = __ldg(next + kB * bank) - a.lv.begin[m];
-      t.end = kB * (bank + 1) < a.lv.count[m - 1] ? __ldg(next + kB * (bank + 1)) - a.lv.begin[m] : a.lv.count[m];
+      t.first = __ldg(next + kBank * bank) - a.lv.begin[m];
+      t.end = kBank * (bank + 1) < a.lv.count[m - 1] ? __ldg(next + kBank * (bank + 1)) - a.lv.begin[m] : a.lv.count[m];
       t.mask = __ldg(a.child_mask[m] + t.first);
       return t;
     };
@@ -622,9 +609,9 @@ __global__ void __launch_bounds__(coarse_threads<TI, kB>(), 2) k_coarse_levels(C
       for (int node = t.first; node < t.end; ++node) {
         unsigned mask = node == t.first ? t.mask : __ldg(a.child_mask[m] + node);
         float v = 0.f;
-        if (mask == (kB == 32 ? kFull : 0xffffu)) {
+        if (mask == kFull) {
 #pragma unroll
-          for (int k = 0; k < kB; ++k) v += c[3 * k + q];
+          for (int k = 0; k < kBank; ++k) v += c[3 * k + q];
         } else {
           for (; mask; mask &= mask - 1u) v += c[3 * (__ffs(mask) - 1) + q];
         }
@@ -637,7 +624,7 @@ __global__ void __launch_bounds__(coarse_threads<TI, kB>(), 2) k_coarse_levels(C
     Parents up[kMaxLevels];
 #pragma unroll
     for (int m = 3; m < kMaxLevels; ++m)
-      if (m <= l && kB * (tid / 3) < sp[m - 1].y - sp[m - 1].x) up[m] = parents(m, sp[m - 1].x / kB + tid / 3);
+      if (m <= l && kBank * (tid / 3) < sp[m - 1].y - sp[m - 1].x) up[m] = parents(m, sp[m - 1].x / kBank + tid / 3);
     float* far = a.scratch;
     for (int m = 3; m < l; ++m) far += coarse_scratch(a.lv, m);
     auto place = [&](int m) {  // where level m's R goes
@@ -650,15 +637,15 @@ __global__ void __launch_bounds__(coarse_threads<TI, kB>(), 2) k_coarse_levels(C
     constexpr int kStride = kN + 4;
     constexpr int kStageBanks = kCoarseStage / kStride < kT / 3 ? kCoarseStage / kStride : kT / 3;
     float* dst = place(2);
-    for (int p = sp[1].x; p < sp[1].y; p += kStageBanks * kB) {
-      const int pe = min(p + kStageBanks * kB, sp[1].y);
+    for (int p = sp[1].x; p < sp[1].y; p += kStageBanks * kBank) {
+      const int pe = min(p + kStageBanks * kBank, sp[1].y);
       const float4* from4 = reinterpret_cast<const float4*>(a.r1 + 3 * (size_t)p);
       const int n4 = (3 * (pe - p) + 3) / 4;  // the arrays are padded to whole 16-byte words
 #pragma unroll 6
       for (int e = tid; e < n4; e += kT) reinterpret_cast<float4*>(stage)[e + e / (kN / 4)] = from4[e];
-      const bool mine = p + kB * (tid / 3) < pe;
+      const bool mine = p + kBank * (tid / 3) < pe;
       Parents t;
-      if (mine) t = parents(2, p / kB + tid / 3);
+      if (mine) t = parents(2, p / kBank + tid / 3);
       __syncthreads();
       if (mine) add_children(2, t, stage + (tid / 3) * kStride, tid % 3, dst, sp[2]);
       __syncthreads();
@@ -667,14 +654,14 @@ __global__ void __launch_bounds__(coarse_threads<TI, kB>(), 2) k_coarse_levels(C
     for (int m = 3; m < kMaxLevels; ++m) {
       if (m > l) break;
       const float* src = dst;
-      const int banks = (sp[m - 1].y - sp[m - 1].x + kB - 1) / kB, bank0 = sp[m - 1].x / kB;
+      const int banks = (sp[m - 1].y - sp[m - 1].x + kBank - 1) / kBank, bank0 = sp[m - 1].x / kBank;
       far += coarse_scratch_level(a.lv, m - 1);
       dst = place(m);
       for (int e = tid; e < 3 * banks; e += kT)
         add_children(m, e == tid ? up[m] : parents(m, bank0 + e / 3), src + (size_t)(e / 3) * kN, e % 3, dst, sp[m]);
       __syncthreads();
     }
-    if (tid >= 3 * min(kB, a.lv.count[l] - (kB * g - a.lv.begin[l])) && tid < kN) xs[tid] = 0.f;
+    if (tid >= 3 * min(kBank, a.lv.count[l] - (kBank * g - a.lv.begin[l])) && tid < kN) xs[tid] = 0.f;
   }
   if constexpr (kTiled) {
     if (tid < kN) vs[tid] = xs[tid] * sc;  // (by the thread that wrote xs[tid], or after its barrier)
@@ -732,8 +719,8 @@ __global__ void __launch_bounds__(coarse_threads<TI, kB>(), 2) k_coarse_levels(C
   } else {
     // the symmetric inverse: block (ln, ln + d) serves both triangles; the
     // products and the order of the sums are those of domain_apply
-    if (d < kD) {
-      const int c = (ln + d) & (kB - 1);
+    if (d < kDiags) {
+      const int c = (ln + d) & (kBank - 1);
       const float x0 = xs[3 * ln], x1 = xs[3 * ln + 1], x2 = xs[3 * ln + 2];
       const float c0 = xs[3 * c], c1 = xs[3 * c + 1], c2 = xs[3 * c + 2];
 #pragma unroll
@@ -746,13 +733,13 @@ __global__ void __launch_bounds__(coarse_threads<TI, kB>(), 2) k_coarse_levels(C
     if (tid < kN) {
       y = p1[tid];
 #pragma unroll
-      for (int q = 1; q < kD; ++q) {
+      for (int q = 1; q < kDiags; ++q) {
         y += p1[kN * q + tid];
         y += p2[kN * q + tid];
       }
     }
   }
-  if (tid < kN) a.z[3 * (size_t)(kB * g - a.c0) + tid] = y;
+  if (tid < kN) a.z[3 * (size_t)(kBank * g - a.c0) + tid] = y;
   if (!pair || !s) return;
   double total = 0.0;
   if (grid_finish<double, kT>(tid < kN ? (double)xs[tid] * y : 0.0, dots, blockIdx.x, gridDim.x,
@@ -783,7 +770,7 @@ CoarseLevels coarse_levels_args(maspcg_handle* h)
 // R of level 1 from the residual on its own (a warp per 32 slots), where no
 // kernel in front summed it: the initial and standalone applies, after a
 // residual replacement, and with the fused x / r update or iteration head.
-template <typename Tv, int kB, bool kFused>
+template <typename Tv, bool kFused>
 __global__ void __launch_bounds__(kTpb) k_restrict1(ApplyArgs a, const Tv* __restrict__ r, PcgScalars* s, FusedArgs fa)
 {
   pdl_wait();
@@ -804,7 +791,7 @@ __global__ void __launch_bounds__(kTpb) k_restrict1(ApplyArgs a, const Tv* __res
       v[2] = (float)rp[2];
     }
   }
-  restrict_bank<kB>(slot < a.c0 ? __ldg(a.cmap1 + slot) : -1, a.coarse_r, v);
+  restrict_bank(slot < a.c0 ? __ldg(a.cmap1 + slot) : -1, a.coarse_r, v);
 }
 
 // The leader of each key group gets the group's sum, its lanes in ascending order.
@@ -1349,13 +1336,10 @@ void build_mas_domains(maspcg_handle* h)
                                                       reinterpret_cast<unsigned*>(h->sort_keys.get()),
                                                       h->sort_vals.get()); MLAUNCHED(h);
     h->perm[l].resize(c0);
-    h->off[l].resize(count + 1);
     size_t tb = h->cub_tmp.cap;
     MCK(cub::DeviceRadixSort::SortPairs(h->cub_tmp.get(), tb, reinterpret_cast<const unsigned*>(h->sort_keys.get()),
                                         reinterpret_cast<unsigned*>(h->sort_keys_out.get()), h->sort_vals.get(),
                                         h->perm[l].get(), c0, 0, bits, st));
-    k_member_offsets<<<ceil_div(h->nv, kTpb), kTpb, 0, st>>>(
-        reinterpret_cast<const unsigned*>(h->sort_keys_out.get()), h->nv, count, h->off[l].get()); MLAUNCHED(h);
   }
   // storage (16-slot banks: FP32 only)
   const int storage = h->bank == 16 ? (int)MASPCG_INV_FP32 : h->cfg.inverse_storage;
@@ -1364,28 +1348,32 @@ void build_mas_domains(maspcg_handle* h)
   if (storage != MASPCG_INV_FP32) h->inv_scale.resize((size_t)lv.domains * 96);
   MCK(cudaMemsetAsync(h->failed.get() + 3, 0, sizeof(int), st));
   launch_factor(h);
-  // children of the coarse nodes and spans below the coarse domains (k_coarse_levels)
   const int coarse_domains = lv.domains - lv.dom_begin[1];
-  size_t below = 0;
-  for (int l = 2; l < lv.levelnum && h->bank == 32; ++l) {
-    h->child_bank[l].resize((size_t)lv.count[l]);
-    h->child_mask[l].resize((size_t)lv.count[l]);
-    k_children<32><<<ceil_div(lv.count[l - 1], kTpb), kTpb, 0, st>>>(h->going_next.get(), lv.begin[l - 1], lv.count[l - 1],
-                                                          lv.begin[l], h->child_bank[l].get(),
-                                                          h->child_mask[l].get());
-    MLAUNCHED(h);
-    below += coarse_scratch(lv, l);
-  }
-  h->coarse_below.resize(std::max<size_t>(below, 1), 4);
-  h->coarse_span.resize((size_t)std::max(coarse_domains, 1) * kMaxLevels);
-  if (coarse_domains > 0 && h->bank == 32) {
-    k_coarse_spans<32><<<ceil_div(coarse_domains, 64), 64, 0, st>>>(
-        coarse_levels_args(h));
-    MLAUNCHED(h);
-  }
   // coarse work vectors (padding entries stay zero)
   const size_t coarse = (size_t)(lv.total_clusters - c0) * 3;
-  h->coarse_r.resize(coarse > 0 ? coarse : 3);
+  if (h->bank == 32) {
+    // children of the coarse nodes and spans below the coarse domains
+    // (k_coarse_levels, which keeps R above level 1 on the chip)
+    size_t below = 0;
+    for (int l = 2; l < lv.levelnum; ++l) {
+      h->child_bank[l].resize((size_t)lv.count[l]);
+      h->child_mask[l].resize((size_t)lv.count[l]);
+      k_children<<<ceil_div(lv.count[l - 1], kTpb), kTpb, 0, st>>>(
+          h->going_next.get(), lv.begin[l - 1], lv.count[l - 1], lv.begin[l], h->child_bank[l].get(),
+          h->child_mask[l].get());
+      MLAUNCHED(h);
+      below += coarse_scratch(lv, l);
+    }
+    h->coarse_below.resize(std::max<size_t>(below, 1), 4);
+    h->coarse_span.resize((size_t)std::max(coarse_domains, 1) * kMaxLevels);
+    h->coarse_r.resize(std::max<size_t>(lv.levelnum > 1 ? 3 * (size_t)(lv.begin[2] - lv.begin[1]) : 0, 3));
+    if (coarse_domains > 0) {
+      k_coarse_spans<<<ceil_div(coarse_domains, 64), 64, 0, st>>>(coarse_levels_args(h));
+      MLAUNCHED(h);
+    }
+  } else {
+    h->coarse_r.resize(std::max<size_t>(coarse, 3));
+  }
   h->coarse_z.resize(coarse > 0 ? coarse : 3);
   h->chain_dot.resize((size_t)std::max(coarse_domains, 1));  // >= CTAs of k16_apply_coarse
   MCK(cudaMemsetAsync(h->coarse_r.get(), 0, h->coarse_r.bytes(), st));
@@ -1497,7 +1485,6 @@ ApplyArgs make_apply_args(maspcg_handle* h)
 {
   ApplyArgs a{};
   a.cmap1 = h->cmap[1].get();
-  a.going_next = h->going_next.get();
   a.coarse_r = h->coarse_r.get();
   a.coarse_z = h->coarse_z.get();
   for (int l = 1; l < h->lv.levelnum && l < kMaxLevels; ++l) a.cmap[l] = h->cmap[l].get();
@@ -1580,17 +1567,17 @@ void level0_apply(maspcg_handle* h, const ApplyArgs& a, int variant, const Tv* r
 
 // The coarse levels on `st`.  fa set: the residual is the fused x / r
 // update's; else restricted says that the kernel in front summed level 1's R.
-template <typename TI, typename Tv, int kB, bool kFused = false>
+template <typename TI, typename Tv, bool kFused = false>
 void launch_coarse(maspcg_handle* h, cudaStream_t st, const ApplyArgs& a, const Tv* r, PcgScalars* s, int mode,
                    int pair, bool restricted, const FusedArgs& fa = FusedArgs{}, int from_level = 1)
 {
   if (kFused || !restricted)
-    launch_pdl_on(h, st, k_restrict1<Tv, kB, kFused>, dim3(ceil_div(h->c0, kTpb)), dim3(kTpb), 0, a, r, s, fa);
+    launch_pdl_on(h, st, k_restrict1<Tv, kFused>, dim3(ceil_div(h->c0, kTpb)), dim3(kTpb), 0, a, r, s, fa);
   if (from_level >= a.lv.levelnum) return;
   constexpr int bytes = (kCoarseStage + 2 * 3 * kCoarseOnChip) * sizeof(float);
-  allow_smem(h, k_coarse_levels<TI, kB>, bytes);
-  launch_pdl_on(h, st, k_coarse_levels<TI, kB>, dim3(a.lv.domains - a.lv.dom_begin[from_level]),
-                dim3(coarse_threads<TI, kB>()), bytes, coarse_levels_args(h), s, mode, pair, h->chain_dot.get());
+  allow_smem(h, k_coarse_levels<TI>, bytes);
+  launch_pdl_on(h, st, k_coarse_levels<TI>, dim3(a.lv.domains - a.lv.dom_begin[from_level]),
+                dim3(coarse_threads<TI>()), bytes, coarse_levels_args(h), s, mode, pair, h->chain_dot.get());
 }
 
 // Whether the overlapped apply takes level 1's domains into the level-0 kernel:
@@ -1624,7 +1611,7 @@ void mas_apply_t(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, int part_b
     return;
   }
   if (!overlap || !s) {
-    launch_coarse<TI, Tv, kBank>(h, h->stream, a, r, s, mode, 0, restricted);
+    launch_coarse<TI, Tv>(h, h->stream, a, r, s, mode, 0, restricted);
     level0_apply<TI, Tv, Tacc>(h, a, variant, r, z, partial, part_base, total_parts, mode, s, grid0);
     return;
   }
@@ -1640,14 +1627,14 @@ void mas_apply_t(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, int part_b
     level0_apply<TI, Tv, Tacc>(h, a, variant, r, z, partial, part_base, total_parts, mode, s, grid0, 0, pair);
   };
   if (level1 && !restricted)
-    launch_pdl(h, k_restrict1<Tv, kBank, false>, dim3(ceil_div(h->c0, kTpb)), dim3(kTpb), 0, a, r, s, FusedArgs{});
+    launch_pdl(h, k_restrict1<Tv, false>, dim3(ceil_div(h->c0, kTpb)), dim3(kTpb), 0, a, r, s, FusedArgs{});
   if (level1 && lv.levelnum == 2) {
     level0(0);
     return;
   }
   MCK(cudaEventRecord(h->ev_fork, h->stream));
   MCK(cudaStreamWaitEvent(h->side_stream, h->ev_fork, 0));
-  launch_coarse<TI, Tv, kBank>(h, h->side_stream, a, r, s, mode, 1, level1 || restricted, FusedArgs{}, level1 ? 2 : 1);
+  launch_coarse<TI, Tv>(h, h->side_stream, a, r, s, mode, 1, level1 || restricted, FusedArgs{}, level1 ? 2 : 1);
   MCK(cudaEventRecord(h->ev_join, h->side_stream));
   level0(1);
   MCK(cudaStreamWaitEvent(h->stream, h->ev_join, 0));
@@ -1673,14 +1660,14 @@ void mas_apply_fused_t(maspcg_handle* h, const FusedArgs& fa, float* z, Tacc* pa
     return;
   }
   if (!overlap) {
-    launch_coarse<TI, float, kBank, true>(h, h->stream, a, nullptr, s, mode, 0, false, fa);
+    launch_coarse<TI, float, true>(h, h->stream, a, nullptr, s, mode, 0, false, fa);
     level0_apply<TI, float, Tacc, true>(h, a, variant, nullptr, z, partial, part_base, total_parts, mode, s, grid0, 1,
                                         0, fa, partial_rr);
     return;
   }
   MCK(cudaEventRecord(h->ev_fork, h->stream));
   MCK(cudaStreamWaitEvent(h->side_stream, h->ev_fork, 0));
-  launch_coarse<TI, float, kBank, true>(h, h->side_stream, a, nullptr, s, mode, 1, false, fa);
+  launch_coarse<TI, float, true>(h, h->side_stream, a, nullptr, s, mode, 1, false, fa);
   MCK(cudaEventRecord(h->ev_join, h->side_stream));
   level0_apply<TI, float, Tacc, true>(h, a, variant, nullptr, z, partial, part_base, total_parts, mode, s, grid0, 0, 1,
                                       fa, partial_rr);
@@ -1738,12 +1725,11 @@ template void mas_apply_fused<double>(maspcg_handle*, const FusedArgs&, float*, 
 // Stage timing helpers: the level-0 domain apply alone, and the domain
 // assembly + inversion alone (member lists from the last build).
 template <typename Tv, typename Tacc>
-void mas_level0_only(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, int grid0, PcgScalars* s, int variant)
+void mas_level0_only(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, PcgScalars* s, int variant)
 {
   ApplyArgs a = make_apply_args(h);
   if (variant < 0) variant = h->apply_variant;
   const int grid = level0_grid(h, variant, false);
-  (void)grid0;
   switch (h->cfg.inverse_storage) {
     case MASPCG_INV_BF16:
       level0_apply<__nv_bfloat16, Tv, Tacc>(h, a, variant, r, z, partial, 0, grid, 0, s, grid);
@@ -1757,10 +1743,9 @@ void mas_level0_only(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, int gr
   }
   MCK(cudaGetLastError());
 }
-template void mas_level0_only<float, float>(maspcg_handle*, const float*, float*, float*, int, PcgScalars*, int);
-template void mas_level0_only<float, double>(maspcg_handle*, const float*, float*, double*, int, PcgScalars*, int);
-template void mas_level0_only<double, double>(maspcg_handle*, const double*, double*, double*, int, PcgScalars*,
-                                              int);
+template void mas_level0_only<float, float>(maspcg_handle*, const float*, float*, float*, PcgScalars*, int);
+template void mas_level0_only<float, double>(maspcg_handle*, const float*, float*, double*, PcgScalars*, int);
+template void mas_level0_only<double, double>(maspcg_handle*, const double*, double*, double*, PcgScalars*, int);
 
 template void mas_apply<float, float>(maspcg_handle*, const float*, float*, float*, int, int, int, int, PcgScalars*,
                                       bool, bool);
@@ -1778,8 +1763,6 @@ template int mas_level0_grid<float, float>(maspcg_handle*, bool);
 template int mas_level0_grid<float, double>(maspcg_handle*, bool);
 template int mas_level0_grid<double, double>(maspcg_handle*, bool);
 
-
-// CTAs of the kernel that completes r.z (level-0 apply or prolongation).
 // CTAs of the level-0 apply, which completes r.z (or part 0 of it).  When
 // the coarse levels run beside it (inside the solve, outside the reference
 // precision) it leaves 16 SMs' worth of CTA slots free: its CTAs take every

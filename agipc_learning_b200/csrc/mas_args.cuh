@@ -10,7 +10,6 @@ struct ApplyArgs {
   const int* cmap1;
   const int* cmap[kMaxLevels];  // fine slot -> level-l local node (-1 padding), l >= 1
   const int* pmr;               // part_map_real: -1 marks a padding slot
-  const int* going_next;
   float* coarse_r;
   float* coarse_z;
   const void* inv;
@@ -49,17 +48,15 @@ __device__ __forceinline__ bool coarse_correction(const ApplyArgs& a, int slot, 
 // accumulated: a butterfly when every bank of the warp is one component (the
 // common case), else the component's lanes in ascending order.  Both orders are
 // fixed.
-template <int kB>
 __device__ __forceinline__ void restrict_bank(int key, float* coarse_r, const float v[3])
 {
   const int lane = threadIdx.x & 31;
   const unsigned grp = __match_any_sync(kFull, key >= 0 ? key : -1 - lane);
-  const unsigned bank = kB == 32 ? kFull : 0xffffu << (lane & 16);
   float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-  if (__all_sync(kFull, grp == bank)) {
+  if (grp == kFull) {
     s0 = v[0], s1 = v[1], s2 = v[2];
 #pragma unroll
-    for (int o = kB / 2; o > 0; o >>= 1) {
+    for (int o = 16; o > 0; o >>= 1) {
       s0 += __shfl_xor_sync(kFull, s0, o);
       s1 += __shfl_xor_sync(kFull, s1, o);
       s2 += __shfl_xor_sync(kFull, s2, o);

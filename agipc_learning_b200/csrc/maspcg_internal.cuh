@@ -215,7 +215,7 @@ struct maspcg_handle {
   maspcg::DBuf<uint32_t> fine_mask, next_mask, next_prefix, next_prefix_sum;
   maspcg::DBuf<int> prefix_orig, prefix_sum_orig, cst, going_next, coarse_table, level_size;
   maspcg::LevelInfo lv{};
-  maspcg::DBuf<int> cmap[maspcg::kMaxLevels], perm[maspcg::kMaxLevels], off[maspcg::kMaxLevels];
+  maspcg::DBuf<int> cmap[maspcg::kMaxLevels], perm[maspcg::kMaxLevels];
   maspcg::DBuf<int> sort_keys, sort_vals, sort_keys_out;
   maspcg::DBuf<unsigned char> cub_tmp;
   maspcg::DBuf<int> scan_tmp;

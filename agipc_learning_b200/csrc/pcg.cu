@@ -30,7 +30,7 @@ void mas_apply(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, int part_bas
                int grid0, PcgScalars* s, bool overlap, bool restricted);
 
 template <typename Tv, typename Tacc>
-void mas_level0_only(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, int grid0, PcgScalars* s, int variant);
+void mas_level0_only(maspcg_handle* h, const Tv* r, Tv* z, Tacc* partial, PcgScalars* s, int variant);
 template <typename Tacc>
 void mas_apply_fused(maspcg_handle* h, const FusedArgs& fa, float* z, Tacc* partial, double* partial_rr, int part_base,
                      int total_parts, int mode, int grid0, PcgScalars* s, bool overlap);
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(kTpb) k_update_xr(Tv* x, Tv* r, const Tv* __re
 // their 96 entries with coalesced accesses (lane, lane + 32, lane + 64), moves
 // the new r to a row per lane with shuffles and restricts it.  Rows outside the
 // MAS range follow.  Spares the coarse levels their pass over r and a launch.
-template <typename Tv, typename Tacc, int kB>
+template <typename Tv, typename Tacc>
 __global__ void __launch_bounds__(kTpb) k_update_xr_restrict(ApplyArgs a, Tv* x, Tv* r, const Tv* __restrict__ p4,
                                                              const Tv* __restrict__ ap, int nrows, int mixed,
                                                              Tacc* partial, PcgScalars* s)
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(kTpb) k_update_xr_restrict(ApplyArgs a, Tv* x,
                   t2 = __shfl_sync(kFull, v[2], e & 31);
       rv[q] = e < 32 ? t0 : (e < 64 ? t1 : t2);
     }
-    restrict_bank<kB>(key, a.coarse_r, rv);
+    restrict_bank(key, a.coarse_r, rv);
   }
   const int lo = 3 * a.fem_off, skip = 3 * a.c0;
   for (int e = blockIdx.x * kTpb + threadIdx.x; e < 3 * nrows - skip; e += gridDim.x * kTpb) {
@@ -1016,9 +1016,8 @@ struct Engine {
       launch_pdl(h, k_update_p<Tv, false>, dim3(grows), dim3(kTpb), 0, a, V(h->vz), V(h->vp4), h->nb_int, s);
     spmv(s);
     if (restricts())
-      launch_pdl(h, k_update_xr_restrict<Tv, Tacc, 32>, dim3(grows),
-                 dim3(kTpb), 0, mas_apply_args(h), V(h->vx), V(h->vr), V(h->vp4), V(h->vap), h->nb_int, mixed ? 1 : 0,
-                 partial(), s);
+      launch_pdl(h, k_update_xr_restrict<Tv, Tacc>, dim3(grows), dim3(kTpb), 0, mas_apply_args(h), V(h->vx),
+                 V(h->vr), V(h->vp4), V(h->vap), h->nb_int, mixed ? 1 : 0, partial(), s);
     else
       launch_pdl(h, k_update_xr<Tv, Tacc>, dim3(grows), dim3(kTpb), 0, V(h->vx), V(h->vr), V(h->vp4), V(h->vap),
                  h->nb_int, mixed ? 1 : 0, partial(), s);
@@ -1271,10 +1270,10 @@ struct Engine {
       switch (stage) {
         case 0: spmv(s); break;
         case 1: precondition(V(h->vr), V(h->vz), 0, s); break;
-        case 2: mas_level0_only<Tv, Tacc>(h, V(h->vr), V(h->vz), partial_rz(), gl0, s, -1); break;
+        case 2: mas_level0_only<Tv, Tacc>(h, V(h->vr), V(h->vz), partial_rz(), s, -1); break;
         case 3: launch_factor(h); break;
         case 7: true_residual(s); break;
-        default: mas_level0_only<Tv, Tacc>(h, V(h->vr), V(h->vz), partial_rz(), gl0, s, stage == 6 ? 0 : stage - 3);
+        default: mas_level0_only<Tv, Tacc>(h, V(h->vr), V(h->vz), partial_rz(), s, stage == 6 ? 0 : stage - 3);
       }
     };
     const bool pdl = h->use_pdl;
