@@ -1,6 +1,8 @@
 """Kernels at the sizes where their tiling can go wrong (ragged tails, row and
 run lengths around a step, one domain, many nodes on one coarse level) against
 the CPU oracle or the mathematics (needs a B200)."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -211,6 +213,65 @@ def test_apply_on_fragmented_hierarchies(n, precision, inverse):
         o.set_inverses(m.domain_inverses())
     zo = o.precondition(s.b)
     assert np.linalg.norm(z - zo) <= 1e-5 * np.linalg.norm(zo)
+
+
+def _with_outer_rows(s, before, after):
+    """The system with rows in front of its FEM range and behind it, each with a
+    diagonal block and one that couples it to an FEM row."""
+    rng = np.random.default_rng(before + after)
+    at = np.concatenate([np.arange(before), before + s.nb + np.arange(after)]).astype(np.int32)
+    fem = before + rng.integers(0, s.nb, len(at)).astype(np.int32)
+    top = np.abs(s.vals).max()
+    vals = np.concatenate([s.vals, np.tile(top * np.eye(3).reshape(1, 9), (len(at), 1)),
+                           0.01 * np.abs(s.vals).mean() * rng.standard_normal((len(at), 9))])
+    return dataclasses.replace(s, nb=s.nb + len(at), fem_offset=before, vals=vals,
+                               rows=np.concatenate([s.rows + before, at, np.minimum(at, fem)]).astype(np.int32),
+                               cols=np.concatenate([s.cols + before, at, np.maximum(at, fem)]).astype(np.int32),
+                               b=np.concatenate([rng.standard_normal(3 * before), s.b, rng.standard_normal(3 * after)]))
+
+
+@pytest.mark.parametrize("precision,inverse", [("reference", "fp32"), ("mixed", "bf16"), ("mixed", "fp32")])
+@pytest.mark.parametrize("n,before,after", [(9, 0, 0), (9, 5, 7), (20, 1, 33)])
+def test_iterates_on_fragmented_hierarchies(n, before, after, precision, inverse):
+    """20 iterations of the solve on banks of many components, with rows outside
+    the FEM range: the fused restriction, the coarse levels beside or before the
+    level-0 apply and r.z from both, against the oracle's iteration with the GPU's
+    own inverses.  1e-5: the bound of one FP32 apply's sums, as above."""
+    s = _with_outer_rows(_islands(n, n), before, after)
+    o = oracle.Mas32.from_system(s)
+    o.reorder(s.pairs)
+    sel = np.nonzero((s.rows >= before) & (s.cols >= before) & (s.rows < before + s.fem_count) &
+                     (s.cols < before + s.fem_count))[0].astype(np.uint32)
+    o.prepare_hessian(s.vals, s.rows, s.cols, sel, before)
+    with MasPcg(precision=precision, inverse=inverse, gate="euclid", tolerance=1e-30, max_iterations=21) as m:
+        _graph(m, s)
+        m.set_matrix(s.vals, s.rows, s.cols, s.nb, before)
+        m.build()
+        o.set_inverses(m.domain_inverses())
+        x, res = m.solve(s.b)
+    xo, ro = oracle.pcg(s.vals, s.rows, s.cols, s.nb, s.b, precond=oracle.PRECOND_MAS32, gate=oracle.GATE_EUCLID,
+                        tol=1e-30, max_iter=21, fem_offset=before, fem_count=s.fem_count, mas=o)
+    assert res["iterations"] == ro["iterations"]
+    assert np.linalg.norm(x - xo) <= 1e-5 * np.linalg.norm(xo)
+
+
+@pytest.mark.parametrize("variant", [0, N.FLAG_APPLY_STAGED2, N.FLAG_APPLY_DIRECT])
+@pytest.mark.parametrize("inverse", ["bf16", "fp32"])
+def test_level_1_beside_level_0(inverse, variant):
+    """A fragmented system large enough that the level-0 kernel takes level 1's
+    domains (2,662 level-0 domains): 20 iterations against the same with the
+    coarse levels on their own, before the level-0 apply.  1e-5: FP32 sums in
+    another order."""
+    s = _islands(44, 3)
+    x = []
+    for flags in (variant, variant | N.FLAG_SEQUENTIAL_COARSE):
+        with MasPcg(precision="mixed", inverse=inverse, gate="euclid", tolerance=1e-30, max_iterations=21,
+                    flags=flags) as m:
+            _graph(m, s)
+            m.set_matrix(s.vals, s.rows, s.cols, s.nb)
+            m.build()
+            x.append(m.solve(s.b)[0])
+    assert np.linalg.norm(x[0] - x[1]) <= 1e-5 * np.linalg.norm(x[1])
 
 
 @pytest.mark.parametrize("inverse", ["bf16", "fp16", "fp32"])
