@@ -544,9 +544,9 @@ constexpr int coarse_threads() { return sizeof(TI) == 2 ? 32 * kTiles16 : kDiags
 // on the chip, loaded before R is needed.  Latency is all that counts here
 // (a few hundred domains of 10-20 KB): a few dependent loads and barriers,
 // where the form before walked up the hierarchy through counters that the CTAs
-// waited on, and one warp applied a domain: 15 us for the 266 coarse domains of
-// the 64^3 system (BF16; 21.9 before), and 31.4 to 28.2 us per iteration at 8,000
-// rows, 53.5 to 43.5 at 64,000, where it is on the critical path.
+// waited on, and one warp applied a domain: 30.7 to 28.2 us per iteration on the
+// 8,000-row system and 50.8 to 44.5 at 64,000 rows with FP16 storage, where it is
+// on the critical path.
 // pair: the level-0 apply runs concurrently and leaves the coarse correction
 // to the p update; this kernel then also sums r.z of the coarse levels, the
 // sum over domains of R.Z (= r . P Z), and completes r.z with the level-0
@@ -1583,11 +1583,12 @@ void launch_coarse(maspcg_handle* h, cudaStream_t st, const ApplyArgs& a, const 
 // Whether the overlapped apply takes level 1's domains into the level-0 kernel:
 // their R is there before it starts, they are the same work, and there are 1/32
 // as many.  Beside it as CTAs of k_coarse_levels they hold the registers of most
-// SMs while its own CTAs wait: 91.6 us per iteration at 262,144 rows, 86.4 this
-// way.  Where the level-0 domains are one round of resident warps no CTA waits
-// and the two ways are equal (28.9 us at 8,000 rows; 44.9 beside it and 45.3 this
-// way at 64,000).  Not where r.z is summed in FP32: the coarse share of it is an
-// FP64 sum.
+// SMs while its own CTAs wait.  Per iteration on cubes in BF16 storage, beside it
+// -> this way: 74,088 rows 45.5 -> 45.6 us, 85,184 49.5 -> 49.8, 97,336 51.5 -> 50.9,
+// 140,608 60.3 -> 58.8, 262,144 84.0 -> 80.5 (91.6 -> 86.4 with 50,000 contacts).
+// The line is where the level-0 domains are more than one round of resident
+// warps, 75,776 rows on 148 SMs; below it no CTA waits and the two ways are equal.
+// Not where r.z is summed in FP32: the coarse share of it is an FP64 sum.
 template <typename Tv, typename Tacc>
 bool takes_level1(const maspcg_handle* h)
 {

@@ -1439,15 +1439,20 @@ double time_stage(maspcg_handle* h, int stage, int repeats)
 // Whether a solve's iterations run as programmatic dependent launches without
 // MASPCG_FLAG_PDL.  In the reference precision the kernels of an iteration are
 // one chain, and the next one's launch and prologue hide behind the last one's
-// tail: 29.5 -> 27.5 us per iteration at 8,000 rows, 47.1 -> 44.0 on the hybrid
-// system (22,000), 75.0 -> 74.4 at 101,565.  Without MAS the chain is the SpMV and
-// two vector updates, and on large systems the waiting CTAs cost more than that
-// (23.5 -> 22.0 us at 21,952 rows, 34.6 -> 37.5 at 64,000).  The overlapped
-// schedule of the other precisions loses by it below 100,000 rows (44.9 -> 48.2 at
-// 64,000) and gains nothing beyond.
+// tail; on large systems the waiting CTAs take room that the running kernel
+// could use.  Per iteration on cubes, without -> with:
+//   MAS32    8,000 rows 29.0 -> 26.8 us, 39,304 40.6 -> 39.8, 110,592 74.7 -> 74.6,
+//            262,144 132.9 -> 131.2
+//   CEMAS16  8,000 32.3 -> 29.4, 39,304 41.2 -> 39.7, 64,000 51.7 -> 50.5,
+//            110,592 67.7 -> 69.6, 175,616 90.2 -> 91.2
+//   no MAS   8,000 19.8 -> 18.2, 27,000 24.1 -> 22.7, 32,768 24.1 -> 23.4, equal from
+//            39,304 on; with many contacts 34.6 -> 37.5 at 64,000
+// The overlapped schedule of the other precisions loses by it below 100,000 rows
+// (44.9 -> 48.2 at 64,000) and gains nothing beyond.
 bool pdl_pays(const maspcg_handle* h)
 {
-  return h->cfg.precision == MASPCG_PREC_REFERENCE && (h->mas_layout || h->nb_int <= 32768);
+  if (h->cfg.precision != MASPCG_PREC_REFERENCE) return false;
+  return !h->mas_layout ? h->nb_int <= 32768 : h->bank == 32 || h->nb_int <= 65536;
 }
 
 struct PdlScope {
