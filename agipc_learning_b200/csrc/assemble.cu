@@ -2,8 +2,8 @@
 //
 // * convert_bcoo: Converter::convert (StiffGIPC/linear_system/utils/
 //   converter.cu:137-284).  Triplets are put in the stable order of (row, col)
-//   by row buckets (rowsort.cu), or, where a row is too long for those, by a
-//   radix sort of the key (row << 32) + col packed into as few bits as the
+//   by row buckets (rowsort.cu), or, where rows are too long or too many for
+//   those, by a radix sort of the key (row << 32) + col packed into as few bits as the
 //   indices need, and each run's 3x3 blocks are summed.  The reference sums a run with
 //   a warp head-segmented reduction plus FP64 atomics, whose order varies;
 //   here each element of a block is summed over its run in the stable sort
@@ -67,7 +67,8 @@ __global__ void k_conv_starts(const int* __restrict__ heads, const int* __restri
 // a block's 72 bytes and write the sum's, so both are coalesced; the runs'
 // entries are fetched four ahead of the sums.  Bound by the latency of the
 // scattered blocks.  On the 110,592-row merge the whole call went from 1.21 to
-// 0.94 ms with this kernel and the range pass above (a thread per key before).
+// 0.94 ms with this kernel and a range pass with fewer atomics (a thread per key
+// before; 0.59 with the row buckets since).
 __global__ void __launch_bounds__(kAsmTpb) k_conv_sum(MergedKeys k, const double* __restrict__ vals,
                                                      int* rows_out, int* cols_out, double* vals_out)
 {

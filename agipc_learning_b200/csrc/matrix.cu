@@ -1,10 +1,11 @@
 // matrix.cu -- assembled BCOO -> internal full BCSR, FP64 SpMV, permutations,
 // block-Jacobi (3x3) and affine-body (12x12) inverses.
 //
-// The conversion follows Converter::convert (converter.cu:137-284): a stable
-// radix sort on a (row,col) key and a segmented sum of equal keys, so the
-// block structure is bit-exact and FP64 sums are taken in input order.  It
-// differs in what it produces: both triangles (the symmetric SpMV of
+// The conversion follows Converter::convert (converter.cu:137-284): the stable
+// order of the (row, col) keys, here by row buckets (rowsort.cu) or, with rows
+// too long or too many for those, by a radix sort, and a segmented sum of equal
+// keys, so the block structure is bit-exact and FP64 sums are taken in input
+// order.  It differs in what it produces: both triangles (the symmetric SpMV of
 // spmv.cu:28-53 scatters B^T with atomics; a row-owned BCSR needs none) and
 // rows renumbered into the MAS partition order.
 #include <algorithm>
@@ -103,8 +104,8 @@ __global__ void k_fill_structure(const unsigned long long* __restrict__ keys, co
 // FP32 tile (null in the reference precision, which does not read it) is
 // transposed in shared memory and written in one run.
 // Bound by the scattered input blocks.  With the row maps formed on the device the
-// matrix of the 64^3 contact system is built in 0.87 ms, 1.31 with a thread per
-// block and the maps copied from the host.
+// matrix of the 64^3 contact system was built in 0.87 ms (0.68 with the row buckets
+// since), 1.31 with a thread per block and the maps copied from the host.
 constexpr int kFillTpb = 288;
 __global__ void __launch_bounds__(kFillTpb) k_fill_values(const int* __restrict__ vals_sorted,
                                                          const int* __restrict__ seg_start, int nnzb, int m_valid,

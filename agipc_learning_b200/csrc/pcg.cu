@@ -1445,8 +1445,8 @@ double time_stage(maspcg_handle* h, int stage, int repeats)
 //            262,144 132.9 -> 131.2
 //   CEMAS16  8,000 32.3 -> 29.4, 39,304 41.2 -> 39.7, 64,000 51.7 -> 50.5,
 //            110,592 67.7 -> 69.6, 175,616 90.2 -> 91.2
-//   no MAS   8,000 19.8 -> 18.2, 27,000 24.1 -> 22.7, 32,768 24.1 -> 23.4, equal from
-//            39,304 on; with many contacts 34.6 -> 37.5 at 64,000
+//   no MAS   8,000 19.8 -> 18.2, 27,000 24.1 -> 22.7, 32,768 24.1 -> 23.4, 35,937
+//            26.3 -> 27.8, 64,000 34.4 -> 37.3
 // The overlapped schedule of the other precisions loses by it below 100,000 rows
 // (44.9 -> 48.2 at 64,000) and gains nothing beyond.
 bool pdl_pays(const maspcg_handle* h)
